@@ -63,8 +63,8 @@ void nekbone_set_mgrid_(const int *ifmgrid);
  * even-odd form in 64-bit fixed point on the integer pipes (default: block
  * floating point, ~55 significant bits of each element's largest value;
  * same result to rounding, ~4x faster on GB300, whose FP64 pipe runs at
- * 1/64 of its FP32 rate).  Odd lx1 falls back to order 0; ax_e_ always uses
- * order 0. */
+ * 1/64 of its FP32 rate).  Form 1 needs an even lx1 and form 2 an even one or
+ * an odd one up to 11; otherwise order 0 runs.  ax_e_ always uses order 0. */
 void nekbone_set_contraction_order_(const int *order);
 /* /cflops/ flop_a, flop_cg (INPUT:8), accumulated as the reference does */
 void nekbone_get_flops_(double *flop_a, double *flop_cg);

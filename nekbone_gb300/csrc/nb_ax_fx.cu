@@ -27,19 +27,22 @@ void decompose(double x, int64_t *m, int *e) {
   *e = ex - 53;
 }
 
-// round((a + sgn b) 2^sh) to the nearest integer (ties to even), from the
-// exact values of a and b (a term below 2^-70 of the other is dropped)
-int64_t scaled_sum(double a, double b, int sgn, int sh) {
-  int64_t ma, mb;
-  int ea, eb;
-  decompose(a, &ma, &ea);
-  decompose(b, &mb, &eb);
-  if (ma == 0) ea = eb;
-  if (mb == 0) eb = ea;
-  if (ea - eb > 70) mb = 0, eb = ea;
-  if (eb - ea > 70) ma = 0, ea = eb;
-  const int e0 = ea < eb ? ea : eb;
-  const i128 T = (i128(ma) << (ea - e0)) + i128(sgn) * (i128(mb) << (eb - e0));
+// round((x[0] + ... + x[nx-1]) 2^sh) to the nearest integer (ties to even),
+// from the exact values (a term below 2^-70 of another is dropped)
+int64_t scaled_sum(const double *x, int nx, int sh) {
+  int64_t m[4];
+  int e[4], top = -100000, e0 = 100000;
+  for (int q = 0; q < nx; ++q) {
+    decompose(x[q], &m[q], &e[q]);
+    if (m[q] != 0) top = std::max(top, e[q]);
+  }
+  for (int q = 0; q < nx; ++q)
+    if (m[q] != 0 && top - e[q] <= 70) e0 = std::min(e0, e[q]);
+    else m[q] = 0;
+  i128 T = 0;
+  for (int q = 0; q < nx; ++q)
+    if (m[q] != 0) T += i128(m[q]) << (e[q] - e0);
+  if (T == 0) return 0;
   const int s = e0 + sh;
   if (s >= 0) return int64_t(T << s);
   if (-s > 120) return 0;
@@ -74,41 +77,80 @@ __global__ void __launch_bounds__(256)
 
 }  // namespace
 
-// E, O of D and of D^T (even_odd_tables' order and meaning) in fixed point
-// with fc fractional bits, |C| <= 2^59, split into balanced halves.
+// The tables of D and of D^T in FxCoef's order and form, with fc fractional
+// bits.
 bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
-               std::vector<int> &lo, int *fc) {
-  if (lx % 2 != 0 || lx < 2) return false;
-  const int h = lx / 2;
-  auto Dm = [&](int r, int c) { return D[r + c * lx]; };
-  double mx = 0.0;
-  for (int a = 0; a < h; ++a)
-    for (int m = 0; m < h; ++m) {
-      mx = std::max(mx, std::fabs(Dm(a, m) + Dm(a, lx - 1 - m)) / 2);
-      mx = std::max(mx, std::fabs(Dm(a, m) - Dm(a, lx - 1 - m)) / 2);
-      mx = std::max(mx, std::fabs(Dm(m, a) + Dm(lx - 1 - m, a)) / 2);
-      mx = std::max(mx, std::fabs(Dm(m, a) - Dm(lx - 1 - m, a)) / 2);
+               std::vector<int> &lo, std::vector<int> &d, int *fc) {
+  // lx1 = 13 and 15 keep the reference's FP64 sums: on random fields this
+  // form's error there is 1.1 to 1.5 times theirs (up to 11 it is smaller)
+  if (lx < 2 || (lx % 2 != 0 && lx > 11)) return false;
+  const int h = lx / 2, h1 = lx - h;
+  const bool full = h1 > h;
+  const int bits = full ? 61 : 59;
+  // value (a, m) of E (even) or O of D or, with tr, of D^T as a sum of terms
+  // over nx: the matrix's entries at (a, m) and (a, n-1-m) and, in the full
+  // form, their mirror images -- subtracted for the main tables (sg = -1),
+  // added for the remainder's (sg = 1)
+  auto terms = [&](bool tr, bool even, int a, int m, int sg, double *x) {
+    auto M = [&](int r, int c) { return tr ? D[c + r * lx] : D[r + c * lx]; };
+    const int s2 = even ? 1 : -1, n1 = lx - 1;
+    const bool mid = full && m == h;  // the middle column: counted once
+    if (!full) {
+      x[0] = M(a, m);
+      x[1] = s2 * M(a, n1 - m);
+      return 2;
     }
+    x[0] = M(a, m);
+    x[1] = sg * M(n1 - a, n1 - m);
+    if (mid) return 2;
+    x[2] = s2 * M(a, n1 - m);
+    x[3] = s2 * sg * M(n1 - a, m);
+    return 4;
+  };
+  double mx = 0.0;
+  for (int tr = 0; tr < 2; ++tr)
+    for (int a = 0; a < h1; ++a)
+      for (int m = 0; m < h1; ++m)
+        for (int even = 0; even < 2; ++even) {
+          if (even ? a >= h : m >= h) continue;
+          double x[4], s = 0.0;
+          const int nx = terms(tr, even, a, m, -1, x);
+          for (int q = 0; q < nx; ++q) s += x[q];
+          mx = std::max(mx, std::fabs(s) / nx);
+        }
   if (!(mx > 0.0)) return false;
   int k = 0;
   std::frexp(mx * (1.0 + 1e-15), &k);  // mx < 2^k
-  *fc = 59 - k;
-  hi.assign(4 * h * h, 0);
-  lo.assign(4 * h * h, 0);
-  auto put = [&](int q, double x1, double x2, int sgn) {
-    const int64_t C = scaled_sum(x1, x2, sgn, *fc - 1);
-    const int32_t l = int32_t(uint32_t(uint64_t(C)));
-    lo[q] = l;
-    hi[q] = int32_t((C - int64_t(l)) >> 32);
-  };
-  for (int a = 0; a < h; ++a)
-    for (int m = 0; m < h; ++m) {
-      put(a * h + m, Dm(a, m), Dm(a, lx - 1 - m), 1);
-      put(h * h + a * h + m, Dm(a, m), Dm(a, lx - 1 - m), -1);
-      put(2 * h * h + a * h + m, Dm(m, a), Dm(lx - 1 - m, a), 1);
-      put(3 * h * h + a * h + m, Dm(m, a), Dm(lx - 1 - m, a), -1);
+  *fc = bits - k;
+  hi.clear();
+  lo.clear();
+  d.clear();
+  bool ok = true;
+  for (int tr = 0; tr < 2; ++tr)
+    for (int even = 1; even >= 0; --even)
+      for (int a = 0; a < (even ? h : h1); ++a)
+        for (int m = 0; m < (even ? h1 : h); ++m) {
+          double x[4];
+          const int nx = terms(tr, even, a, m, -1, x);
+          const int64_t C = scaled_sum(x, nx, *fc - (nx == 4 ? 2 : 1));
+          const int32_t l = int32_t(uint32_t(uint64_t(C)));
+          lo.push_back(l);
+          hi.push_back(int32_t((C - int64_t(l)) >> 32));
+        }
+  if (!full) return true;
+  for (int tr = 0; tr < 2; ++tr)
+    for (int even = 1; even >= 0; --even) {
+      const int nr = even ? h1 : h;
+      for (int a = 0; a < nr; ++a)
+        for (int m = 0; m < nr; ++m) {
+          double x[4];
+          const int nx = terms(tr, even, a, m, 1, x);
+          const int64_t C = scaled_sum(x, nx, *fc - (nx == 4 ? 2 : 1));
+          if (C > (1 << 28) || C < -(1 << 28)) ok = false;
+          d.push_back(int(C));
+        }
     }
-  return true;
+  return ok;
 }
 
 void metric_fx_invalidate(const Operator &op) { op.gfx_src = nullptr; }

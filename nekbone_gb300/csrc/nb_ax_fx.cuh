@@ -39,6 +39,9 @@
 //    exact move of the exponent field; the input goes in by an exact FP64
 //    scaling and the FP64-to-integer conversion (two more), where the FP64
 //    pipe has room beside the integer work.
+// Odd lx1 up to 11 takes a form with more bits (FxCoef): 50 CG iterations on
+// 12 x 10 x 9 elements at lx1 = 9 in 4.28 ms instead of 9.07 with the
+// reference-order operator on the FP64 pipe.
 // This is block floating point: the error of a value is bounded relative to
 // the largest value of its element (~2^-56), where FP64 bounds it relative
 // to the value itself.  Results agree with the reference's FP64 evaluation
@@ -84,22 +87,40 @@ __device__ __forceinline__ Sp split(i64 x) {
   return s;
 }
 
-// A sum of products a*b in units of 2^64: hh counts ah*bh, x and x2 count
+// A sum of products a*b in units of 2^(64-K): hh counts ah*bh, x and x2 count
 // ah*bl and al*bh in units of 2^32 (two accumulators: two dependency chains
 // of half the length), x started at half a unit so that the high word of
 // x + x2 rounds to nearest (al*bl dropped).  Each product is one 32x32 ->
 // 64-bit multiply-add (mad.wide.s32), written in C++ so that a coefficient
-// can stay a constant-bank operand.
+// can stay a constant-bank operand.  For the three terms of the metric step;
+// K = 2 keeps two more bits of its outputs.
+template <int K>
 struct Acc {
   i64 hh, x, x2;
-  __device__ __forceinline__ Acc() : hh(0), x(1ll << 31), x2(0) {}
-  __device__ __forceinline__ void mac(int chi, int clo, const Sp &v) {
+  __device__ __forceinline__ Acc() : hh(0), x(1ll << (31 - K)), x2(0) {}
+  __device__ __forceinline__ void mac(const Sp &c, const Sp &v) {
+    hh += i64(c.hi) * i64(v.hi);
+    x += i64(c.hi) * i64(v.lo);
+    x2 += i64(c.lo) * i64(v.hi);
+  }
+  __device__ __forceinline__ i64 result() const { return (hh << K) + ((x + x2) >> (32 - K)); }
+};
+
+// The same (K = 0) for the up to six terms of the FULL form's lines, |c| <=
+// 2^61 and |v| <= 2^62: the al*bh of even and odd terms go to two
+// accumulators, so that each sum stays within 64 bits (three terms of at most
+// 2^61, six of at most 2^60), each rounded to units of 2^64.
+struct AccF {
+  i64 hh, x, x2[2];
+  __device__ __forceinline__ AccF() : hh(0), x(1ll << 31), x2{1ll << 31, 1ll << 31} {}
+  __device__ __forceinline__ void mac(int chi, int clo, const Sp &v, int m) {
     hh += i64(chi) * i64(v.hi);
     x += i64(chi) * i64(v.lo);
-    x2 += i64(clo) * i64(v.hi);
+    x2[m & 1] += i64(clo) * i64(v.hi);
   }
-  __device__ __forceinline__ void mac(const Sp &c, const Sp &v) { mac(c.hi, c.lo, v); }
-  __device__ __forceinline__ i64 result() const { return hh + ((x + x2) >> 32); }
+  __device__ __forceinline__ i64 result(int) const {
+    return hh + ((x >> 32) + ((x2[0] >> 32) + (x2[1] >> 32)));
+  }
 };
 
 // The same sum with the two cross terms taken as high words only: each
@@ -118,7 +139,7 @@ struct AccH {
   int x, x2;  // high words below 2^27 (|ah| < 2^28, |al| <= 2^31); the
               // lx1/2 <= 8 of them and x + x2 stay below 2^31
   __device__ __forceinline__ AccH() : hh(0), x(0), x2(0) {}
-  __device__ __forceinline__ void mac(int chi, int clo, const Sp &v) {
+  __device__ __forceinline__ void mac(int chi, int clo, const Sp &v, int) {
     hh += i64(chi) * i64(v.hi);
     x = __mulhi(chi, v.lo) + x;
     x2 = __mulhi(clo, v.hi) + x2;
@@ -130,9 +151,10 @@ struct AccH {
 };
 
 // v * 2^sh for 0 <= sh < 64: the operator's two renormalisation shifts are
-// never negative.  After the gradient every output is below 2^58.6 (six
+// never negative (values below 2^59; the FULL form has two bits more
+// everywhere).  After the gradient every output is below 2^59 (lx1
 // products of |C| <= 2^59 and an even-odd sum below 2^60, in units of 2^64,
-// twice), so its shift is >= 0; after the metric step every output is below
+// lx1 <= 16), so its shift is >= 0; after the metric step every output is below
 // 2^56.6 (three products of |G| < 2^60 and a value below 2^59), so its shift
 // is >= 2.  The operator checks both and reports a violation through the
 // device error word.
@@ -222,16 +244,38 @@ __device__ __forceinline__ unsigned warp_mask(int nt, int w) {
 }
 
 // ------------------------------------------------------------ operator --
-// Derivative tables in fixed point: E, O of D, then E, O of D^T (the
-// even-odd tables of k_ax_eo, 4*(lx1/2)^2 values, row a), as balanced
-// halves, |coefficient| <= 2^59.  A kernel parameter, read as multiply-add
-// operands.
+// Derivative tables in fixed point, as balanced halves.  With h = lx1/2 and
+// h1 = lx1 - h, the anti-centrosymmetric part of a matrix (D, then D^T) is E,
+// h rows of h1 values, and O, h1 rows of h (row a):
+//   y(a) = E ve + O vo,  y(n-1-a) = O vo - E ve;
+// for odd lx1 the middle value of a line, its own mirror image, joins the
+// sums (last column of E) and the middle output, which the antisymmetry
+// leaves to the differences alone, the differences (last row of O).
+//
+// Even lx1 (FxCoef::FULL false): |coefficient| <= 2^59, |line value| < 2^59,
+// cross terms as high words (AccH); the matrix's other part, the rounding
+// (~1e-15) by which D misses the symmetry, is dropped.
+// Odd lx1 up to 11 (FULL): these orders' other form is the reference's own
+// FP64 sums, and this one is to be no less exact: |coefficient| <= 2^61 and
+// |line value| < 2^61, cross terms in full (AccF), and the centrosymmetric
+// remainder of D kept as one 32-bit coefficient more a product, in the unit
+// of lo (dE, h1 rows of h1 values, and dO, h rows of h):
+//   y(a) += dE ve + dO vo,  y(n-1-a) += dE ve - dO vo.
+// A kernel parameter, read as multiply-add operands.
 template <int LX>
 struct FxCoef {
-  int hi[4 * (LX / 2) * (LX / 2)];
-  int lo[4 * (LX / 2) * (LX / 2)];
+  static constexpr int H = LX / 2, H1 = LX - H;
+  static constexpr bool FULL = LX % 2 != 0;
+  static constexpr int Q = 4 * H * H1;                       // main values, D and D^T
+  static constexpr int QD = FULL ? 2 * (H1 * H1 + H * H) : 1;  // remainders
+  int hi[Q];
+  int lo[Q];
+  int d[QD];
   int fc;  // fractional bits: coefficient = (hi 2^32 + lo) 2^-fc
 };
+// bits of a line's values: |v| < 2^kLine (and of a block after renormalising)
+template <int LX>
+constexpr int fx_bits() { return FxCoef<LX>::FULL ? 61 : 59; }
 
 template <int LX>
 struct FxShared {
@@ -253,31 +297,55 @@ __device__ __forceinline__ int fx_at(int i, int j, int k) {
   return i + LX * j + (LX * LX + 1) * k;
 }
 
-// y(0..n-1) = C v of one line v (fixed point, |v| < 2^59), coefficient
-// tables at offset q0 of cf (E at q0, O at q0 + h^2); y in units of 2^64 of
-// the products (|y| < 2^58.6), handed to put(m, y(m)) as soon as each pair
-// y(a), y(n-1-a) is formed (no output array stays live)
+// y(0..n-1) = C v of one line v (fixed point, |v| < 2^fx_bits), matrix tr of
+// cf (0 D, 1 D^T); y in units of 2^64 of the products, handed to put(m,
+// y(m)) as soon as each pair y(a), y(n-1-a) is formed (no output array stays
+// live).  |y| < 2^59 (2^60 in the FULL form: the rows of D and of D^T sum to
+// at most three times the largest coefficient).
 template <int LX, typename Put>
-__device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int q0, Put put) {
-  constexpr int H = LX / 2;
-  Sp ve[H], vo[H];
+__device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int tr, Put put) {
+  constexpr int H = LX / 2, H1 = LX - H;
+  constexpr bool FULL = FxCoef<LX>::FULL;
+  typedef typename std::conditional<FULL, AccF, AccH>::type A;
+  const int qe0 = tr * 2 * H * H1, qo0 = qe0 + H * H1;
+  const int de0 = tr * (H1 * H1 + H * H), do0 = de0 + H1 * H1;
+  Sp ve[H1], vo[H];
 #pragma unroll
   for (int m = 0; m < H; ++m) {
     ve[m] = split(v[m] + v[LX - 1 - m]);
     vo[m] = split(v[m] - v[LX - 1 - m]);
   }
+  if constexpr (H1 > H) ve[H1 - 1] = split(v[H]);
   NB_FX_UNROLL(NB_FX_AUNROLL)
   for (int a = 0; a < H; ++a) {
-    AccH e, o;
+    A e, o;
 #pragma unroll
-    for (int m = 0; m < H; ++m) {
-      const int qe = q0 + a * H + m, qo = qe + H * H;
-      e.mac(cf.hi[qe], cf.lo[qe], ve[m]);
-      o.mac(cf.hi[qo], cf.lo[qo], vo[m]);
+    for (int m = 0; m < H1; ++m) e.mac(cf.hi[qe0 + a * H1 + m], cf.lo[qe0 + a * H1 + m], ve[m], m);
+#pragma unroll
+    for (int m = 0; m < H; ++m) o.mac(cf.hi[qo0 + a * H + m], cf.lo[qo0 + a * H + m], vo[m], m);
+    const i64 ye = e.result(H1), yo = o.result(H);
+    if constexpr (FULL) {
+      i64 ze = 0, zo = 0;
+#pragma unroll
+      for (int m = 0; m < H1; ++m) ze += i64(cf.d[de0 + a * H1 + m]) * i64(ve[m].hi);
+#pragma unroll
+      for (int m = 0; m < H; ++m) zo += i64(cf.d[do0 + a * H + m]) * i64(vo[m].hi);
+      put(a, ye + yo + ((ze + zo) >> 32));
+      put(LX - 1 - a, yo - ye + ((ze - zo) >> 32));
+    } else {
+      put(a, ye + yo);
+      put(LX - 1 - a, yo - ye);
     }
-    const i64 ye = e.result(H), yo = o.result(H);
-    put(a, ye + yo);
-    put(LX - 1 - a, yo - ye);
+  }
+  if constexpr (FULL) {  // the middle output
+    A o;
+    i64 ze = 0;
+#pragma unroll
+    for (int m = 0; m < H; ++m)
+      o.mac(cf.hi[qo0 + H * H + m], cf.lo[qo0 + H * H + m], vo[m], m);
+#pragma unroll
+    for (int m = 0; m < H1; ++m) ze += i64(cf.d[de0 + H * H1 + m]) * i64(ve[m].hi);
+    put(H, o.result(H) + (ze >> 32));
   }
 }
 
@@ -292,12 +360,13 @@ __device__ __forceinline__ void fx_or_post(u64 v, unsigned *orl, unsigned *orh, 
     orh[w] = h;
   }
 }
-// the shift that brings the block's largest magnitude below 2^59
-__device__ __forceinline__ int fx_or_shift(const unsigned *orl, const unsigned *orh, int nt) {
+// the shift that brings the block's largest magnitude below 2^bits
+__device__ __forceinline__ int fx_or_shift(const unsigned *orl, const unsigned *orh, int nt,
+                                           int bits) {
   u64 v = 0;
   for (int w = 0; w < (nt + 31) / 32; ++w) v |= (u64(orh[w]) << 32) | orl[w];
   if (v == 0) return 0;
-  return 58 - (63 - __clzll(i64(v)));
+  return bits - 1 - (63 - __clzll(i64(v)));
 }
 // one's complement magnitude: the same top bit as |v| (one lower for an
 // exact negative power of two, which the bounds leave room for)
@@ -309,7 +378,7 @@ template <int LX, int MODE>
 __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef<LX> &cf) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FxShared<LX> &sm = *reinterpret_cast<FxShared<LX> *>(smem_raw);
-  constexpr int L2 = LX * LX, L3 = LX * LX * LX, H = LX / 2;
+  constexpr int L2 = LX * LX, L3 = LX * LX * LX, BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 2 : 0;
   const int t = threadIdx.x + LX * threadIdx.y;
   const int i = threadIdx.x, j = threadIdx.y;  // own column (i,j)
   const int e = blockIdx.x;
@@ -357,9 +426,9 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     em = 0;
     for (int q = 0; q < (L2 + 31) / 32; ++q) em = max(em, sm.emax[q]);
 #pragma unroll
-    for (int k = 0; k < LX; ++k) sm.A[fx_at<LX>(i, j, k)] = to_fixed_cvt(uk[k], em, 6);
+    for (int k = 0; k < LX; ++k) sm.A[fx_at<LX>(i, j, k)] = to_fixed_cvt(uk[k], em, BITS - 53);
   }
-  const int sP = em - 1081;  // p = P 2^sP
+  const int sP = em - 1075 - (BITS - 53);  // p = P 2^sP
   __syncthreads();
 
   // Thread (i,j) takes, in each contraction stage, the r-line (j, k=i),
@@ -388,7 +457,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   }
   fx_or_post(orv, sm.orl, sm.orh, t, L2);
   __syncthreads();
-  int s1 = fx_or_shift(sm.orl, sm.orh, L2);
+  int s1 = fx_or_shift(sm.orl, sm.orh, L2, BITS);
   if (s1 < 0) {  // outside the bounds shift_up relies on: results invalid
     if (t == 0 && a.err) atomicOr(a.err, 2u);
     s1 = 0;
@@ -397,7 +466,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
 
   // metric (cg.f:156-163) at the thread's own points, in place
   const int eg = a.gexp[e];
-  const int sW = 64 + (eg - 1082) + sU;  // wr = WR 2^sW before renormalising
+  const int sW = 64 - MK + (eg - 1082) + sU;  // wr = WR 2^sW before renormalising
   orv = 0;
 #pragma unroll 4
   for (int k = 0; k < LX; ++k) {
@@ -408,7 +477,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
     const Sp G1 = {g01.x, g01.y}, G2 = {g01.z, g01.w}, G3 = {g23.x, g23.y},
              G4 = {g23.z, g23.w}, G5 = {g45.x, g45.y}, G6 = {g45.z, g45.w};
-    Acc wr, ws, wt;
+    Acc<MK> wr, ws, wt;
     wr.mac(G1, ur); wr.mac(G2, us); wr.mac(G3, ut);
     ws.mac(G2, ur); ws.mac(G4, us); ws.mac(G5, ut);
     wt.mac(G3, ur); wt.mac(G5, us); wt.mac(G6, ut);
@@ -420,7 +489,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   }
   fx_or_post(orv, sm.orl, sm.orh, t, L2);
   __syncthreads();
-  int s2 = fx_or_shift(sm.orl, sm.orh, L2);
+  int s2 = fx_or_shift(sm.orl, sm.orh, L2, BITS);
   if (s2 < 0) {  // as s1
     if (t == 0 && a.err) atomicOr(a.err, 2u);
     s2 = 0;
@@ -438,7 +507,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     i64 v[LX];
 #pragma unroll
     for (int m = 0; m < LX; ++m) v[m] = shift_up(src[b0 + m * st], s2);
-    fx_line<LX>(v, cf, 2 * H * H, [&](int m, i64 y) { out[b0 + m * st] = y; });
+    fx_line<LX>(v, cf, 1, [&](int m, i64 y) { out[b0 + m * st] = y; });
   }
   __syncthreads();
 

@@ -1178,7 +1178,7 @@ int batch_build(Batch *B, int nprob, const int *nx, const int *ny, const int *nz
     op->lx = L;
     op->n = G.n;
     op->nelt = G.nel;
-    op->fx_ok = fx_tables(d, L, op->FXhi, op->FXlo, &op->fx_fc);
+    op->fx_ok = fx_tables(d, L, op->FXhi, op->FXlo, op->FXd, &op->fx_fc);
     if (op->fx_ok) G.fx = op;
     // default shape: the first listed (the even-odd form where lx1 is even)
     const auto s32 = batch_shapes_f32(L);

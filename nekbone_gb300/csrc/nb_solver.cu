@@ -127,8 +127,7 @@ int CgWork::ensure(const Operator &op, int niter) {
 }
 
 // ------------------------------------------------------------ set-up --
-bool even_odd_tables(const std::vector<double> &D, int lx, std::vector<double> &eo) {
-  if (lx % 2 != 0) return false;
+bool anti_centrosymmetric(const std::vector<double> &D, int lx) {
   double dmax = 0.0, asym = 0.0;
   auto Dm = [&](int r, int c) { return D[r + c * lx]; };
   for (int r = 0; r < lx; ++r)
@@ -136,7 +135,12 @@ bool even_odd_tables(const std::vector<double> &D, int lx, std::vector<double> &
       dmax = std::max(dmax, std::fabs(Dm(r, c)));
       asym = std::max(asym, std::fabs(Dm(r, c) + Dm(lx - 1 - r, lx - 1 - c)));
     }
-  if (asym > 1e-12 * dmax) return false;
+  return asym <= 1e-12 * dmax;
+}
+
+bool even_odd_tables(const std::vector<double> &D, int lx, std::vector<double> &eo) {
+  if (lx % 2 != 0 || !anti_centrosymmetric(D, lx)) return false;
+  auto Dm = [&](int r, int c) { return D[r + c * lx]; };
   const int h = lx / 2;
   eo.assign(4 * h * h, 0.0);
   for (int a = 0; a < h; ++a)
@@ -371,7 +375,8 @@ int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
   NB_CUDA(cudaMemcpy(op->fD, fDh.data(), lx * lx * sizeof(float), cudaMemcpyHostToDevice));
   // even-odd tables when D(n-1-i,n-1-m) = -D(i,m) holds to rounding
   op->eo_ok = even_odd_tables(op->D, lx, op->EO);
-  op->fx_ok = op->eo_ok && fx_tables(op->D, lx, op->FXhi, op->FXlo, &op->fx_fc);
+  op->fx_ok = anti_centrosymmetric(op->D, lx) &&
+              fx_tables(op->D, lx, op->FXhi, op->FXlo, op->FXd, &op->fx_fc);
   op->face.resize(nelt);
   for (int e = 0; e < nelt; ++e)
     op->face[e] = (unsigned char)face_bits(op->lglel[e], nelx, nely, nelz);

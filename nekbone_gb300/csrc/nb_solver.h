@@ -25,7 +25,7 @@ struct Operator {
   bool eo_ok = false;
   // the same tables in fixed point for the FP64 operator on the integer
   // pipes (nb_ax_fx.cuh): balanced halves, fx_fc fractional bits
-  std::vector<int> FXhi, FXlo;
+  std::vector<int> FXhi, FXlo, FXd;
   int fx_fc = 0;
   bool fx_ok = false;
   // the metric of the solve in progress in fixed point (metric_fx_prepare):
@@ -36,9 +36,9 @@ struct Operator {
   mutable const double *gfx_src = nullptr;
   mutable long gfx_cap = 0;
   int order = 2;                   // 0 reference left-to-right sums, 1 even-odd
-                                   // (FP64 and FP32 operators alike), 2 (default)
-                                   // the FP64 operator in fixed point where the
-                                   // even-odd tables exist (FP32: even-odd)
+                                   // (FP64 and FP32 operators alike, even lx1),
+                                   // 2 (default) the FP64 operator in fixed point,
+                                   // odd lx1 up to 11 too (FP32: as 1)
   GsHost gsh_host;                 // jl maps of the dssum handle
   GsDevice gs;                     // device form
   // mask state (maskit, cg.f:214-258)
@@ -107,13 +107,16 @@ int operator_box(Operator *op, int nelx, int nely, int nelz, int lx,
 int operator_from(Operator *op, int nelx, int nely, int nelz, int nelt,
                   int lx, const int *lglel, const double *dxm1,
                   const GsHost &maps, int mask_mode, cudaStream_t s);
+// Whether D(n-1-i,n-1-m) = -D(i,m) to rounding, as the GLL derivative
+bool anti_centrosymmetric(const std::vector<double> &D, int lx);
 // E, O of D and of D^T (4*(lx/2)^2 values) when lx is even and D is
 // anti-centrosymmetric to rounding (the even-odd contraction form).
 bool even_odd_tables(const std::vector<double> &D, int lx, std::vector<double> &eo);
-// The even-odd tables in fixed point (nb_ax_fx.cu): balanced 32-bit halves of
-// round(C 2^fc), |round(C 2^fc)| <= 2^59, from D's exact values.
+// The even-odd tables in fixed point (nb_ax_fx.cu; FxCoef's form): balanced
+// 32-bit halves of round(C 2^fc) from D's exact values and, for odd lx, the
+// remainders d.
 bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
-               std::vector<int> &lo, int *fc);
+               std::vector<int> &lo, std::vector<int> &d, int *fc);
 // The metric g in the fixed-point operator's form, converted when g is not
 // the array last converted (one pass over g); metric_fx_invalidate forgets
 // the conversion (every solve and every standalone apply starts with it, so
