@@ -1072,7 +1072,7 @@ int nb_pcg_tol(nb_mesh *mesh, double *x, const double *f, const double *g,
   MgPrecond M(mesh->mg.get());
   int done = 0, stt = NB_OK;
   double rn0 = 0.0, rn = 0.0;
-  stt = cg_begin(op, wk, x, f, c, r, max_iter, s);
+  stt = cg_begin(op, wk, x, f, c, r, max_iter, true, s);
   if (!stt && cudaMemcpy(&rn0, &wk.sc->rnorm, 8, cudaMemcpyDeviceToHost) != cudaSuccess)
     stt = fail(NB_ERR_CUDA, "nb_pcg_tol: reading rnorm");
   rn = rn0;

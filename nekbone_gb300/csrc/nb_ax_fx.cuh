@@ -511,29 +511,39 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   }
   __syncthreads();
 
-  // w_L = tr + ts + tt in FP64; the CG epilogue as k_ax_eo's.  The
-  // interior's p (written above by this thread, so in cache), c and f are
-  // read again here rather than held in registers through the contractions.
+  // w_L = tr + ts + tt in FP64; the CG epilogue as k_ax_eo's.  p (written
+  // above by this thread, so in cache), c and f are read again here rather
+  // than held in registers through the contractions.
+  const bool whole = MODE == 1 && box_flag(a.box_ok);  // pap formed here (BoxMesh)
+  const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
   const bool col_interior = (i > 0) && (i < LX - 1) && (j > 0) && (j < LX - 1);
+  // an element with a value that is not finite has no fixed-point form
+  const bool bad = em == 0x7FF || eg == 0x7FF;
   double part = 0.0;
   double pk[LX], ck[LX], fk[LX];
-  if (MODE != 0 && col_interior) {
+  if (MODE != 0 && (col_interior || whole)) {
 #pragma unroll
-    for (int k = 1; k < LX - 1; ++k) {  // all loads before the first store
+    for (int k = 0; k < LX; ++k) {  // all loads before the first store
       const size_t id = base + size_t(k) * L2 + t;
-      pk[k] = a.p[id];
-      ck[k] = __ldg(a.c + id);
-      if (MODE == 2) fk[k] = __ldg(a.f + id);
+      const bool interior = col_interior && k > 0 && k < LX - 1;
+      if (interior || whole) pk[k] = a.p[id];
+      if (interior && !whole) ck[k] = __ldg(a.c + id);
+      if (MODE == 2 && interior) fk[k] = __ldg(a.f + id);
     }
   }
 #pragma unroll
   for (int k = 0; k < LX; ++k) {
     const int q = fx_at<LX>(i, j, k);
     double wl = to_double_cvt(sm.A[q] + sm.C[q] + sm.D[q], sT);
+    if (bad) wl = __longlong_as_double(0x7FF8000000000000ll);
     const size_t id = base + size_t(k) * L2 + t;
     const bool interior = col_interior && (k > 0) && (k < LX - 1);
     if (MODE == 1) {
-      if (interior) {
+      if (whole) {
+        const double wv = fma_rn(box_tenth<double>(box_ext<LX>(i, j, k) & nbr), pk[k], wl);
+        part = fma_rn(wv, pk[k], part);
+        if (interior) wl = wv;
+      } else if (interior) {
         wl = fma_rn(0.1, pk[k], wl);
         part = fma_rn(mul_rn(wl, ck[k]), pk[k], part);
       }

@@ -90,8 +90,115 @@ struct CgScalars {
   double rtr_first;  // rtr of iteration 1 (cg.f:68)
   double alpha_prev;  // alpha of the iteration whose x update was deferred
   int iter;
-  int pad;
+  int box_ok;         // this solve takes the assembled update (BoxMesh)
 };
+
+// -------------------------------------------------------- assembled update --
+// A brick box (lglel(e) = e): the copies of a point are known in closed form,
+// 2^m of them, m the number of its extreme local indices on element faces
+// with a neighbour.  There a CG iteration needs no pass that writes the
+// gather-scatter sums back: the update reads each boundary point's copies of
+// w_L itself (in jl's order, so every copy forms the same sum), and, since
+// then p is equal at all copies of a point,
+//   pap = sum_points c p (sum over copies of w_L + 0.1 p)
+//       = sum over every local point of p (w_L + 0.1 c p),
+// which the element operator sums as it makes w_L.  Measured: boundary pass
+// and update at 32^3, lx1 = 12, FP64: 0.406 + 0.476 -> 0.007 + 0.533 ms; FP32
+// at 24^3: 0.115 + 0.077 -> 0.007 + 0.105 ms.
+// k_box_begin checks what that takes, once per solve: c is 2^-m bitwise at
+// every point, and r is equal at all unmasked copies of every point (a masked
+// copy has w = r = p = 0).  Where it does not hold the flag stays 0 and the
+// iteration is the general one.
+struct BoxMesh {
+  int nx, ny, nz;            // elements per direction; nx = 0: not a brick box
+  int lx;
+  const unsigned char *face;  // the elements' faces on the domain boundary (box_ext's bits)
+  int full_mask;             // 1: every domain face masked; 0: mask0
+  const unsigned char *mask0;  // mask of element 0's points (no other element's)
+  const unsigned *bnd;         // the nbnd boundary points of an element, l | ext << 16,
+  int nbnd;                    //   faces first, then edges, then corners
+};
+// bits of the local indices that are extreme: 0/1 i = 0 / lx-1, 2/3 j, 4/5 k
+__device__ __forceinline__ unsigned box_ext(int i, int j, int k, int lx) {
+  return (i == 0 ? 1u : 0u) | (i == lx - 1 ? 2u : 0u) | (j == 0 ? 4u : 0u) |
+         (j == lx - 1 ? 8u : 0u) | (k == 0 ? 16u : 0u) | (k == lx - 1 ? 32u : 0u);
+}
+template <int LX>
+__device__ __forceinline__ unsigned box_ext(int i, int j, int k) {
+  return box_ext(i, j, k, LX);
+}
+// the faces of element e that have a neighbour, in the same bits (read, not
+// computed: with three index divisions a point k_box_begin took 0.178 instead
+// of 0.107 ms, FP32 at 24^3)
+__device__ __forceinline__ unsigned box_neighbours(const BoxMesh &b, int e) {
+  return 63u & ~unsigned(__ldg(b.face + e));
+}
+__device__ __forceinline__ bool box_same(double a, double b) {
+  return __double_as_longlong(a) == __double_as_longlong(b);
+}
+__device__ __forceinline__ bool box_same(float a, float b) {
+  return __float_as_int(a) == __float_as_int(b);
+}
+__device__ __forceinline__ bool box_flag(const int *ok) { return ok && *ok; }
+// 2^-m, exactly, m the set bits of nb
+template <typename T>
+__device__ __forceinline__ T box_mult(unsigned nb) {
+  if constexpr (sizeof(T) == 8)
+    return T(__hiloint2double((1023 - __popc(nb)) << 20, 0));
+  else
+    return T(__int_as_float((127 - __popc(nb)) << 23));
+}
+// 0.1 * 2^-m (exact: a power of two times the constant)
+template <typename T>
+__device__ __forceinline__ T box_tenth(unsigned nb) {
+  if constexpr (sizeof(T) == 8) {
+    const double t = 0.1;
+    return T(__hiloint2double(__double2hiint(t) - (__popc(nb) << 20), __double2loint(t)));
+  } else {
+    return T(__int_as_float(__float_as_int(0.1f) - (__popc(nb) << 23)));
+  }
+}
+// Whether point l (extreme bits ext) of element e (faces nbr) is masked.
+__device__ __forceinline__ bool box_masked(const BoxMesh &b, int e, int l, unsigned ext,
+                                           unsigned nbr) {
+  return b.full_mask ? (ext & ~nbr) != 0u : (e == 0 && b.mask0[l] != 0);
+}
+// The copies of a local point q (n < 2^31): q0 the lowest, and the distances
+// to the others along each direction (0: no copy there).
+struct BoxCopies {
+  int q0, d0, d1, d2;
+};
+__device__ __forceinline__ BoxCopies box_copies(const BoxMesh &b, int q, unsigned nb) {
+  const int lx = b.lx, n1 = lx - 1, l3 = lx * lx * lx;
+  BoxCopies c;
+  c.d0 = (nb & 3u) ? l3 - n1 : 0;
+  c.d1 = (nb & 12u) ? l3 * b.nx - n1 * lx : 0;
+  c.d2 = (nb & 48u) ? l3 * b.nx * b.ny - n1 * lx * lx : 0;
+  c.q0 = q - ((nb & 1u) ? c.d0 : 0) - ((nb & 4u) ? c.d1 : 0) - ((nb & 16u) ? c.d2 : 0);
+  return c;
+}
+// Sum of w over the copies, left to right in ascending order (jl's:
+// gather_T_add, jl/gs_local.c:60-75).
+template <typename T>
+__device__ __forceinline__ T box_sum(const T *__restrict__ w, const BoxCopies &c) {
+  T t = w[c.q0];
+  if (c.d0) t = add_rn(t, w[c.q0 + c.d0]);
+  if (c.d1) {
+    const T a = w[c.q0 + c.d1], b = c.d0 ? w[c.q0 + c.d0 + c.d1] : T(0);
+    t = add_rn(t, a);
+    if (c.d0) t = add_rn(t, b);
+  }
+  if (c.d2) {
+    const int q = c.q0 + c.d2;
+    const T a = w[q], b = c.d0 ? w[q + c.d0] : T(0), d = c.d1 ? w[q + c.d1] : T(0),
+            f = c.d0 && c.d1 ? w[q + c.d0 + c.d1] : T(0);
+    t = add_rn(t, a);
+    if (c.d0) t = add_rn(t, b);
+    if (c.d1) t = add_rn(t, d);
+    if (c.d0 && c.d1) t = add_rn(t, f);
+  }
+  return t;
+}
 
 // ------------------------------------------------------------ ax kernel --
 // MODE 0: w = A_L u for every point (the element loop of ax, cg.f:111-114).
@@ -133,6 +240,8 @@ struct AxArgs {
   int act_stride;      //   problem is no longer active); null for one mesh
   int c_unit_interior;  // MODE 1: c is 1 at every element-interior point (a
                         //   verified multiplicity): not read there
+  BoxMesh box;         // MODE 1, with box_ok (the solve's flag; null: general form):
+  const int *box_ok;   //   partial is the element's whole part of pap
 };
 
 template <typename T, int LX>
@@ -366,6 +475,49 @@ constexpr size_t ax_smem_bytes() {
   return sizeof(AxShared<T, LX>);
 }
 
+// ------------------------------------------------- assembled update's pap --
+// pap = the sum of the elements' partials, alpha = rtz1 / pap, by the first
+// blocks of the boundary pass's grid (256 partials each).  With element 0's
+// own mask (the reference's list) a masked copy has p = 0 while the others of
+// its point do not: those few points' terms are replaced.
+template <typename T>
+__device__ __forceinline__ void box_alpha(const T *w, const T *p, double *partial,
+                                          const double *ax_partial, int n, unsigned *counter,
+                                          CgScalars *sc, const BoxMesh &box, double *red) {
+  const int nb = min(int(gridDim.x), (n + int(blockDim.x) - 1) / int(blockDim.x));
+  if (int(blockIdx.x) >= nb) return;
+  double v = 0.0;
+  for (int q = blockIdx.x * blockDim.x + threadIdx.x; q < n; q += nb * blockDim.x)
+    v += ax_partial[q];
+  double pap = block_sum<double>(v, red);
+  if (nb > 1) {
+    if (threadIdx.x == 0) partial[blockIdx.x] = pap;
+    if (!last_block(counter, nb)) return;
+    pap = block_sum_array(partial, nb, red);
+  }
+  if (!box.full_mask) {
+    const int lx = box.lx, l3 = lx * lx * lx;
+    const unsigned nbr = box_neighbours(box, 0);
+    double d = 0.0;
+    for (int l = threadIdx.x; l < l3; l += blockDim.x) {
+      const unsigned cp = box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx) & nbr;
+      if (!cp || !box.mask0[l]) continue;
+      const BoxCopies c = box_copies(box, l, cp);
+      const double t = double(box_sum(w, c)), cm = box_mult<double>(cp);
+      const double pv = double(p[c.q0 + c.d0 + c.d1 + c.d2]);
+      const double others = double((1 << __popc(cp)) - 1);
+      // all but element 0's copy: c p (t + 0.1 p) instead of p (w_L + 0.1 c p)
+      d += others * cm * pv * t - pv * (t - double(w[l]));
+    }
+    __syncthreads();
+    pap += block_sum<double>(d, red);
+  }
+  if (threadIdx.x == 0) {
+    sc->pap = pap;
+    sc->alpha = sc->rtz1 / pap;
+  }
+}
+
 // ------------------------------------------------ gather-scatter finish --
 // For every group of element-boundary points: t = sum of w_L over the group
 // in jl's member order (gather_T_add, jl/gs_local.c:60-75); each member gets
@@ -385,8 +537,13 @@ __global__ void __launch_bounds__(256, NB_GS_MINB)
              const T *__restrict__ c, const int *__restrict__ off,
              const unsigned *__restrict__ idx, int ng,
              double *__restrict__ partial, const double *__restrict__ ax_partial,
-             int n_ax_partial, unsigned *counter, CgScalars *sc) {
+             int n_ax_partial, unsigned *counter, CgScalars *sc, const BoxMesh box,
+             const int *box_ok) {
   __shared__ double red[32];
+  if (box_flag(box_ok)) {  // the assembled update: only pap and alpha are left
+    box_alpha(w, p, partial, ax_partial, n_ax_partial, counter, sc, box, red);
+    return;
+  }
   T part = T(0);
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng;
        g += gridDim.x * blockDim.x) {
@@ -646,6 +803,234 @@ __global__ void __launch_bounds__(256)
         sc->rtz1 = rtr;
         sc->beta = sc->rtz1 / sc->rtz2;
       }
+    }
+  }
+}
+
+// r c for c = 2^-m: the exponent moved instead of a multiplication on the
+// FP64 pipe (a value too small to hold it has no square above zero either, so
+// the sum of r c r is the same)
+__device__ __forceinline__ double box_scale(double r, int m) {
+  const int hi = __double2hiint(r);
+  return ((hi >> 20) & 0x7FF) > m ? __hiloint2double(hi - (m << 20), __double2loint(r)) : 0.0;
+}
+__device__ __forceinline__ float box_scale(float r, int m) {
+  return mul_rn(r, __int_as_float((127 - m) << 23));
+}
+
+// k_cg_update with the sums over copies and the mask taken here (BoxMesh).
+// A block takes an element at a time: first its boundary points, w = sum of
+// w_L over the copies + 0.1 p (0 when masked), into shared memory; then every
+// point as k_cg_update, c formed.  The boundary points come from a table
+// sorted by kind (faces, edges, corners): on GB300 an FP64 instruction costs
+// its warp the same whether one lane or all take part (two lanes a cycle and
+// SM), and the one-pass form, in which every warp holds a few boundary
+// points, took 1.33 ms at 32^3 (this one 0.40 / 0.66 ms for the two halves of
+// a pair; the FP64 pipe and HBM bound it).
+// Where the solve's flag is off, w is already finished and this is
+// k_cg_update's loop.  VEC points a thread at a time (16 bytes) when every
+// vector is aligned and lx1 is even, else one.
+// (eight blocks per SM, 32 registers: 0.53 ms for the pair's average at 32^3
+// FP64 and 0.105 ms at 24^3 FP32, against 0.53 and 0.121 with five)
+template <typename T, int DEFER, int VEC>
+__global__ void __launch_bounds__(256, 8)
+    k_cg_update_box(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p,
+                    const T *__restrict__ w, const T *__restrict__ c, long n,
+                    double *__restrict__ partial, unsigned *counter, CgScalars *sc,
+                    double *hist, int iter, const T *__restrict__ pprev, const BoxMesh box) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[32];
+  struct alignas(VEC * sizeof(T)) Pack { T v[VEC]; };
+  const bool whole = sc->box_ok != 0;
+  const int lx = box.lx, l3 = lx * lx * lx;
+  T *wb = reinterpret_cast<T *>(smem_raw);           // l3: w of the boundary points
+  unsigned char *ext = smem_raw + l3 * sizeof(T);    // l3: extreme bits
+  const T alpha = T(sc->alpha);
+  const T alphm = -alpha;
+  const T alpha0 = DEFER == 2 ? T(sc->alpha_prev) : T(0);
+  if (DEFER == 1 && blockIdx.x == 0 && threadIdx.x == 0) sc->alpha_prev = sc->alpha;
+  T part = T(0);
+  // one pack of points: x and r updated, c r r added
+  auto update = [&](unsigned v, const Pack &wa, const Pack &xa_, const Pack &pa, const Pack &qa,
+                    Pack ra, const int *m, const Pack *ca) {
+    Pack xa = xa_;
+#pragma unroll
+    for (int q = 0; q < VEC; ++q) {
+      if (DEFER == 2) xa.v[q] = fma_rn(alpha0, qa.v[q], xa.v[q]);
+      if (DEFER != 1) xa.v[q] = fma_rn(alpha, pa.v[q], xa.v[q]);
+      ra.v[q] = fma_rn(alphm, wa.v[q], ra.v[q]);
+      const T rc = ca ? mul_rn(ra.v[q], ca->v[q]) : box_scale(ra.v[q], m[q]);
+      part = fma_rn(rc, ra.v[q], part);
+    }
+    if (DEFER != 1) reinterpret_cast<Pack *>(x)[v] = xa;
+    reinterpret_cast<Pack *>(r)[v] = ra;
+  };
+  if (whole) {
+    for (int l = threadIdx.x; l < l3; l += blockDim.x)
+      ext[l] = (unsigned char)box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx);
+    const int Q = l3 / VEC, nelt = int(n / l3);
+    for (int e = blockIdx.x; e < nelt; e += gridDim.x) {
+      const unsigned nbr = box_neighbours(box, e);
+      const int base = e * l3;
+      // faces: one copy at most besides the point's own, no branches
+      const int nf = 6 * (lx - 2) * (lx - 2);
+#pragma unroll 3
+      for (int b = threadIdx.x; b < nf; b += blockDim.x) {
+        const unsigned u = __ldg(box.bnd + b);
+        const int l = int(u & 0xFFFFu);
+        const unsigned ex = u >> 16, cp = ex & nbr;
+        const BoxCopies c = box_copies(box, base + l, cp);
+        const int d = c.d0 + c.d1 + c.d2;
+        const T pv = p[base + l], a = w[c.q0], o = w[c.q0 + d];
+        const T t = fma_rn(T(0.1), pv, d ? add_rn(a, o) : a);
+        wb[l] = box_masked(box, e, l, ex, nbr) ? T(0) : t;
+      }
+      for (int b = nf + threadIdx.x; b < box.nbnd; b += blockDim.x) {
+        const unsigned u = __ldg(box.bnd + b);
+        const int l = int(u & 0xFFFFu);
+        const unsigned ex = u >> 16, cp = ex & nbr;
+        const bool masked = box_masked(box, e, l, ex, nbr);
+        T t = T(0);
+        if (!masked) t = fma_rn(T(0.1), p[base + l], box_sum(w, box_copies(box, base + l, cp)));
+        wb[l] = t;
+      }
+      __syncthreads();
+      const int v0 = base / VEC;
+      for (int v = threadIdx.x; v < Q; v += blockDim.x) {
+        Pack xa, ra, pa, wa, qa;
+        int m[VEC];
+        if (DEFER != 1) {
+          xa = reinterpret_cast<const Pack *>(x)[v0 + v];
+          pa = reinterpret_cast<const Pack *>(p)[v0 + v];
+        }
+        if (DEFER == 2) qa = reinterpret_cast<const Pack *>(pprev)[v0 + v];
+        ra = reinterpret_cast<const Pack *>(r)[v0 + v];
+        wa = reinterpret_cast<const Pack *>(w)[v0 + v];
+        const Pack ba = reinterpret_cast<const Pack *>(wb)[v];
+#pragma unroll
+        for (int q = 0; q < VEC; ++q) {
+          const unsigned ex = ext[v * VEC + q];
+          m[q] = __popc(ex & nbr);
+          if (ex) wa.v[q] = ba.v[q];
+        }
+        update(unsigned(v0 + v), wa, xa, pa, qa, ra, m, nullptr);
+      }
+      __syncthreads();
+    }
+  } else {
+    const unsigned nv = unsigned(n / VEC), vs = gridDim.x * blockDim.x;
+    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += vs) {
+      Pack xa, ra, pa, wa, ca, qa;
+      if (DEFER != 1) {
+        xa = reinterpret_cast<const Pack *>(x)[v];
+        pa = reinterpret_cast<const Pack *>(p)[v];
+      }
+      if (DEFER == 2) qa = reinterpret_cast<const Pack *>(pprev)[v];
+      ra = reinterpret_cast<const Pack *>(r)[v];
+      wa = reinterpret_cast<const Pack *>(w)[v];
+      ca = reinterpret_cast<const Pack *>(c)[v];
+      update(v, wa, xa, pa, qa, ra, nullptr, &ca);
+    }
+  }
+  const double s = block_sum<T>(part, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (last_block(counter, gridDim.x)) {
+    const double rtr = block_sum_array(partial, gridDim.x, red);
+    if (threadIdx.x == 0) {
+      sc->rtr = rtr;
+      if (iter == 1) sc->rtr_first = rtr;
+      sc->rnorm = sqrt(rtr);
+      sc->iter = iter;
+      if (hist) {
+        double *h = hist + 5 * iter;
+        h[0] = sc->rnorm;
+        h[1] = sc->alpha;
+        h[2] = sc->beta;
+        h[3] = sc->pap;
+        h[4] = sc->rtz1;
+      }
+      sc->rtz2 = sc->rtz1;
+      sc->rtz1 = rtr;
+      sc->beta = sc->rtz1 / sc->rtz2;
+    }
+  }
+}
+
+// The start of a solve on a box (cg.f:36-42): x = 0, r = mask(f), rnorm, and
+// whether the assembled update holds (BoxMesh); sc->box_ok is set before and
+// cleared here.  f may be r itself.  One pass instead of a memset, a copy, a
+// mask and a glsc3.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_box_begin(T *x, const T *f, T *r, const T *c, long n, double *__restrict__ partial,
+                unsigned *counter, CgScalars *sc, double *hist, const BoxMesh box) {
+  __shared__ double red[32];
+  __shared__ unsigned char ext[4096];
+  const int lx = box.lx, l3 = lx * lx * lx;
+  for (int l = threadIdx.x; l < l3; l += blockDim.x)
+    ext[l] = (unsigned char)box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx);
+  __syncthreads();
+  const unsigned q0 = blockIdx.x * blockDim.x + threadIdx.x, qs = gridDim.x * blockDim.x;
+  int e = int(q0 / l3), l = int(q0 % l3);
+  const int se = int(qs / l3), sl = int(qs % l3);
+  T part = T(0);
+  bool ok = true;
+  for (long q = q0; q < n; q += qs) {
+    const unsigned nbr = box_neighbours(box, e), ex = ext[l], cp = ex & nbr;
+    const T fv = f[q], cv = c[q];
+    const bool masked = ex && box_masked(box, e, l, ex, nbr);
+    const T rv = masked ? T(0) : fv;
+    // (bitwise, on the integer pipe: a zero of the other sign takes the
+    // general iteration)
+    ok &= box_same(cv, box_mult<T>(cp));
+    if ((cp & 42u) && !masked) {  // against the copies above (none is element 0's)
+      const BoxCopies d = box_copies(box, int(q), cp);
+      if (cp & 2u) ok &= box_same(fv, f[q + d.d0]);
+      if (cp & 8u) ok &= box_same(fv, f[q + d.d1]);
+      if (cp & 32u) ok &= box_same(fv, f[q + d.d2]);
+    }
+    if (x) x[q] = T(0);
+    r[q] = rv;
+    part = fma_rn(mul_rn(rv, cv), rv, part);
+    l += sl;
+    e += se;
+    if (l >= l3) {
+      l -= l3;
+      ++e;
+    }
+  }
+  if (!__syncthreads_and(ok) && threadIdx.x == 0) atomicExch(&sc->box_ok, 0);
+  const double s = block_sum<T>(part, red);
+  if (threadIdx.x == 0) partial[blockIdx.x] = s;
+  if (last_block(counter, gridDim.x)) {
+    const double v = block_sum_array(partial, gridDim.x, red);
+    if (threadIdx.x == 0) {
+      sc->rnorm = sqrt(v);
+      sc->rtz1 = v;   // with z = r the first rtz1 equals this value
+      sc->rtz2 = 1.0;
+      sc->beta = 0.0;
+      if (hist) {
+        hist[0] = sc->rnorm;
+        hist[1] = hist[2] = hist[3] = hist[4] = 0.0;
+      }
+    }
+  }
+}
+
+// After a solve's last assembled update: w finished at the boundary points,
+// as the boundary pass leaves it.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_box_finish(T *__restrict__ w, const T *__restrict__ p, const int *__restrict__ off,
+                 const unsigned *__restrict__ idx, int ng, const int *box_ok) {
+  if (!box_flag(box_ok)) return;
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
+    const int b = off[g], e = off[g + 1];
+    T t = w[idx[b] & 0x7fffffffu];
+    for (int q = b + 1; q < e; ++q) t = add_rn(t, w[idx[q] & 0x7fffffffu]);
+    for (int q = b; q < e; ++q) {
+      const unsigned m = idx[q], id = m & 0x7fffffffu;
+      w[id] = (m & 0x80000000u) ? T(0) : fma_rn(T(0.1), p[id], t);
     }
   }
 }
@@ -1068,6 +1453,8 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
       ureg[k] = a.u[id];
     }
   }
+  // (after the element's loads: nothing waits for the flag before them)
+  const bool whole = sizeof(T) == 4 && MODE == 1 && box_flag(a.box_ok);  // pap formed here
 #pragma unroll
   for (int k = 0; k < LX; ++k) {
     const size_t id = base + size_t(k) * L2 + t;
@@ -1148,6 +1535,7 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
   __syncthreads();
 
   T part = T(0);
+  const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
 #pragma unroll
   for (int k = 0; k < LX; ++k) {
     const int q = eo_at<T, LX>(i, j, k);
@@ -1155,7 +1543,11 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
     const size_t id = base + size_t(k) * L2 + t;
     const bool interior = col_interior && (k > 0) && (k < LX - 1);
     if (MODE == 1) {
-      if (interior) {
+      if (whole) {
+        const T wv = fma_rn(box_tenth<T>(box_ext<LX>(i, j, k) & nbr), ureg[k], wl);
+        part = fma_rn(wv, ureg[k], part);
+        if (interior) wl = wv;
+      } else if (interior) {
         wl = fma_rn(T(0.1), ureg[k], wl);
         part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);
       }

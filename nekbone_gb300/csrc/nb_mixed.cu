@@ -161,7 +161,7 @@ int nb_cg_tol(nb_mesh *mesh, double *x, const double *f, const double *g,
   double rn0 = 0, rn = 0;
   // run CG in chunks: cg_device always starts from x=0, so iterate one long
   // solve with the device scalars and poll rnorm every check_every steps.
-  int st = cg_begin(op, wk, x, f, c, r, max_iter, s);
+  int st = cg_begin(op, wk, x, f, c, r, max_iter, false, s);
   if (!st) {
     NB_CUDA(cudaMemcpyAsync(&rn0, &wk.sc->rnorm, 8, cudaMemcpyDeviceToHost, s));
     NB_CUDA(cudaStreamSynchronize(s));
@@ -304,7 +304,7 @@ int nb_cg_mixed(nb_mesh *mesh, double *x, const double *f, const double *g,
     wk.c32_face = closed ? cface : nullptr;
     if (!st)
       st = cg_device_f32(op, wk, e32, r32, g32, c32, rr32, w32, p32, inner_iters, s,
-                         g_paired_update ? p32b : nullptr);
+                         g_paired_update ? p32b : nullptr, false);
     wk.g32_uniform = 0;
     wk.tc_inner = false;
     wk.c32_face = nullptr;

@@ -8,6 +8,8 @@
 //                   w = sum + 0.1 p, Dirichlet mask, boundary part of pap;
 //                   last block forms pap and alpha
 //   k_cg_update     x += alpha p, r -= alpha w, rtr; last block forms beta
+// On a brick box (BoxMesh) the operator sums all of pap, k_gs_fin only forms
+// alpha from it, and k_cg_update_box takes the sums over copies itself.
 // CG scalars stay on the device.  The unfused path (element product, jl
 // gather-scatter, add2s2, maskit, glsc3 as separate kernels) covers meshes
 // whose numbering shares element-interior points, and flagged handles.
@@ -30,6 +32,23 @@ Operator::~Operator() {
   if (bnd_idx) cudaFree(bnd_idx);
   if (gfx) cudaFree(gfx);
   if (gexp) cudaFree(gexp);
+  if (d_mask0) cudaFree(d_mask0);
+  if (d_bnd_pts) cudaFree(d_bnd_pts);
+}
+
+BoxMesh Operator::box_mesh() const {
+  BoxMesh b{};
+  if (!box_groups || !fused_ok || !mask_built || (mask_mode != 1 && !mask0_ok)) return b;
+  b.nx = nelx;
+  b.ny = nely;
+  b.nz = nelz;
+  b.lx = lx;
+  b.face = d_face;
+  b.full_mask = mask_mode == 1 ? 1 : 0;
+  b.mask0 = d_mask0;
+  b.bnd = d_bnd_pts;
+  b.nbnd = n_bnd_pts;
+  return b;
 }
 
 CgWork::~CgWork() {
@@ -274,6 +293,42 @@ static void build_boundary_groups(Operator *op) {
   op->fused_ok = n < (1L << 31);
 }
 
+// Whether every boundary group (build_boundary_groups) is the brick box's
+// copies of a point: elements in brick order, members ascending.
+static bool is_box_groups(const Operator &op) {
+  if (!op.fused_ok || op.nelt != op.nelx * op.nely * op.nelz) return false;
+  for (int e = 0; e < op.nelt; ++e)
+    if (op.lglel[e] != e + 1) return false;
+  const int lx = op.lx, n1 = lx - 1;
+  const long l3 = long(lx) * lx * lx, ex = op.nelx, ey = op.nely;
+  for (int g = 0; g < op.nbg; ++g) {
+    const int b = op.bnd_off_h[g], m = op.bnd_off_h[g + 1] - b;
+    const long q = op.bnd_idx_h[b], e = q / l3;
+    const int l = int(q % l3), i = l % lx, j = (l / lx) % lx, k = l / (lx * lx);
+    // the group's first member is its lowest copy: the others lie above it
+    const bool up[3] = {i == n1 && e % ex < ex - 1, j == n1 && e / ex % ey < ey - 1,
+                        k == n1 && e / (ex * ey) < op.nelz - 1};
+    if ((i == 0 && e % ex > 0) || (j == 0 && e / ex % ey > 0) || (k == 0 && e / (ex * ey) > 0))
+      return false;
+    const long d[3] = {l3 - n1, l3 * ex - long(n1) * lx, l3 * ex * ey - long(n1) * lx * lx};
+    int at = 0;
+    for (int c = 0; c < 8; ++c) {
+      long o = q;
+      bool in = true;
+      for (int a = 0; a < 3; ++a)
+        if (c >> a & 1) {
+          in = in && up[a];
+          o += d[a];
+        }
+      if (!in) continue;
+      if (at >= m || long(op.bnd_idx_h[b + at]) != o) return false;
+      ++at;
+    }
+    if (at != m) return false;
+  }
+  return true;
+}
+
 namespace {
 // Mask flags of boundary-group members built on the device: bit 31 set
 // exactly for the members in the sorted list (binary search).
@@ -323,6 +378,15 @@ int operator_set_mask(Operator *op, const std::vector<int> &list_in) {
     NB_CUDA(cudaMalloc(&op->d_mask_list, list.size() * sizeof(int)));
     NB_CUDA(cudaMemcpy(op->d_mask_list, list.data(), list.size() * sizeof(int),
                        cudaMemcpyHostToDevice));
+  }
+  op->mask0_ok = false;
+  const int l3 = op->lx * op->lx * op->lx;
+  if (op->box_groups && op->mask_mode == 0 && (list.empty() || list.back() < l3)) {
+    std::vector<unsigned char> m0(l3, 0);
+    for (int v : list) m0[v] = 1;
+    if (!op->d_mask0) NB_CUDA(cudaMalloc(&op->d_mask0, l3));
+    NB_CUDA(cudaMemcpy(op->d_mask0, m0.data(), l3, cudaMemcpyHostToDevice));
+    op->mask0_ok = true;
   }
   if (op->nbg > 0 && op->bnd_idx_h.empty() && op->bnd_idx) {
     // groups built on the device (nb_topo.cu): flags set there
@@ -377,6 +441,22 @@ int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
   op->eo_ok = even_odd_tables(op->D, lx, op->EO);
   op->fx_ok = anti_centrosymmetric(op->D, lx) &&
               fx_tables(op->D, lx, op->FXhi, op->FXlo, op->FXd, &op->fx_fc);
+  // an element's boundary points, one face, edge or corner after the other
+  std::vector<unsigned> of[64], pts;
+  for (int l = 0; l < lx * lx * lx; ++l) {
+    const int v[3] = {l % lx, (l / lx) % lx, l / (lx * lx)};
+    unsigned ex = 0;
+    for (int a = 0; a < 3; ++a)
+      ex |= (v[a] == 0 ? 1u : 0u) << (2 * a) | (v[a] == lx - 1 ? 1u : 0u) << (2 * a + 1);
+    if (ex) of[ex].push_back(unsigned(l) | ex << 16);
+  }
+  for (int kind = 1; kind <= 3; ++kind)
+    for (int f = 1; f < 64; ++f)
+      if (__builtin_popcount(f) == kind) pts.insert(pts.end(), of[f].begin(), of[f].end());
+  op->n_bnd_pts = int(pts.size());
+  NB_CUDA(cudaMalloc(&op->d_bnd_pts, pts.size() * sizeof(unsigned)));
+  NB_CUDA(cudaMemcpy(op->d_bnd_pts, pts.data(), pts.size() * sizeof(unsigned),
+                     cudaMemcpyHostToDevice));
   op->face.resize(nelt);
   for (int e = 0; e < nelt; ++e)
     op->face[e] = (unsigned char)face_bits(op->lglel[e], nelx, nely, nelz);
@@ -392,6 +472,7 @@ int operator_from(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
   op->gsh_host = maps;
   NB_TRY(gs_upload(op->gsh_host, int(op->n), &op->gs, s));
   build_boundary_groups(op);
+  op->box_groups = is_box_groups(*op);
   op->mask_built = false;
   if (mask_mode == 1) {
     op->mask_built = true;
@@ -544,12 +625,48 @@ int c_closed_form(const Operator &op, const float *c32, unsigned char *cface, in
 }
 
 namespace {
-// k_cg_update with pairing mode D; FP32 forms c in closed form when the
-// solve in progress verified it (wk.c32_face)
+// the resident blocks of k_cg_update_box: its grid is one wave
+template <typename T, int D, int VEC>
+int update_box_blocks(int lx, int nt, size_t sm) {
+  static int cached[kMaxLx + 1] = {0};
+  if (!cached[lx]) {
+    int b = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_update_box<T, D, VEC>, nt, sm);
+    cached[lx] = sm_count() * std::max(1, b);
+  }
+  return cached[lx];
+}
+
+// The third kernel of an iteration, pairing mode D: the assembled update on
+// a box; else k_cg_update, FP32 with c in closed form when the solve in
+// progress verified it (wk.c32_face)
 template <typename T, int D>
 void update_launch(const Operator &op, const CgWork &wk, T *x, T *r, const T *p,
                    const T *w, const T *c, double *hist, int iter, int identity,
                    float *r32, const T *pprev, cudaStream_t s) {
+  if (wk.box.nx > 0) {
+    constexpr int VEC = 16 / int(sizeof(T));
+    const uintptr_t al = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(r) |
+                         reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(w) |
+                         reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(pprev);
+    // threads: as many as take the element's packs in equal turns of at most 256
+    const bool vec = (al & 15u) == 0 && op.lx % 2 == 0;
+    const int l3 = op.lx * op.lx * op.lx, Q = vec ? l3 / VEC : l3;
+    const int nt = std::max(32, (Q / ((Q + 255) / 256) + 31) / 32 * 32);
+    const size_t sm = size_t(l3) * (sizeof(T) + 1);
+    const int grid = std::min(std::min(wk.grid_up, std::max(op.nelt, 1)),
+                              vec ? update_box_blocks<T, D, VEC>(op.lx, nt, sm)
+                                  : update_box_blocks<T, D, 1>(op.lx, nt, sm));
+    if (vec)
+      k_cg_update_box<T, D, VEC><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
+                                                      wk.counters + 1, wk.sc, hist, iter,
+                                                      pprev, wk.box);
+    else
+      k_cg_update_box<T, D, 1><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
+                                                    wk.counters + 1, wk.sc, hist, iter, pprev,
+                                                    wk.box);
+    return;
+  }
   if constexpr (std::is_same<T, float>::value) {
     if (wk.c32_face) {
       k_cg_update<T, D, true><<<wk.grid_up, 256, 0, s>>>(
@@ -660,19 +777,45 @@ template int apply_ax<double>(const Operator &, double *, const double *, const 
 template int apply_ax<float>(const Operator &, float *, const float *, const float *, cudaStream_t);
 
 // ------------------------------------------------------------------ CG --
-// cg.f:36-42: x = 0, r = mask(f), rnorm = sqrt(glsc3(r,c,r)).
+// Whether an unpreconditioned solve in T on op may take the assembled update:
+// a box, and the element operator that sums pap over every point (the
+// fixed-point FP64 one, the even-odd FP32 one).
+template <typename T>
+static bool box_form(const Operator &op) {
+  if (op.box_mesh().nx == 0) return false;
+  return std::is_same<T, double>::value ? op.order == 2 && op.fx_ok : op.order >= 1 && op.eo_ok;
+}
+
+// cg.f:36-42: x = 0, r = mask(f), rnorm = sqrt(glsc3(r,c,r)).  plain: the
+// solve runs the fused iteration without preconditioner.
 template <typename T>
 static int cg_begin_t(Operator &op, CgWork &wk, T *x, const T *f, const T *c,
-                      T *r, bool zero_x, int niter, cudaStream_t s) {
+                      T *r, bool plain, int niter, cudaStream_t s) {
   const long n = op.n;
   NB_TRY(wk.ensure(op, niter));
   wk.r32_ready = false;
+  wk.box = BoxMesh{};
   if (std::is_same<T, double>::value) metric_fx_invalidate(op);
-  if (zero_x) NB_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));  // rzero(x)
-  NB_TRY(vec_copy<T>(r, f, n, s));                                 // copy(r,f)
-  NB_TRY(maskit_dev<T>(op, r, s));
-  return vec_glsc3<T>(r, c, r, n, wk, wk.dot_out, wk.sc, 1, 0, s);
+  // the reference's list is built by its first mask (of r, below)
+  const bool built = op.mask_built || op.mask_mode == 1;
+  if (!built || !plain || !box_form<T>(op)) {
+    NB_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));  // rzero(x)
+    NB_TRY(vec_copy<T>(r, f, n, s));                   // copy(r,f)
+    NB_TRY(maskit_dev<T>(op, r, s));
+    if (!plain || !box_form<T>(op))
+      return vec_glsc3<T>(r, c, r, n, wk, wk.dot_out, wk.sc, 1, 0, s);
+    f = r;
+  }
+  wk.box = op.box_mesh();
+  NB_CUDA(cudaMemsetAsync(&wk.sc->box_ok, 1, sizeof(int), s));
+  k_box_begin<T><<<wk.grid_up, 256, 0, s>>>(f == r ? nullptr : x, f, r, c, n, wk.partial_up,
+                                            wk.counters + 1, wk.sc, wk.hist, wk.box);
+  NB_CUDA(cudaGetLastError());
+  return NB_OK;
 }
+
+// the flag of the solve begun, for the kernels that act on it
+static const int *box_ok(const CgWork &wk) { return wk.box.nx > 0 ? &wk.sc->box_ok : nullptr; }
 
 // iterations it0..it1 of cg.f:48-75.  With p_alt (the fused, unpreconditioned
 // iteration), the directions of odd iterations go to p and those of even
@@ -684,6 +827,8 @@ static int cg_steps_t(Operator &op, CgWork &wk, T *x, const T *g, const T *c,
                       T *r, T *w, T *p, T *z, int it0, int it1, int niter,
                       Precond *M, bool force_unfused, cudaStream_t s,
                       T *p_alt = nullptr) {
+  if (wk.box.nx > 0 && (M || force_unfused || (std::is_same<T, float>::value && wk.tc_inner)))
+    return fail(NB_ERR_STATE, "cg: a solve begun for the assembled update");
   const long n = op.n;
   const T *D = std::is_same<T, double>::value ? (const T *)op.dD : (const T *)op.fD;
   const bool tc = std::is_same<T, float>::value && wk.tc_inner;
@@ -729,10 +874,13 @@ static int cg_steps_t(Operator &op, CgWork &wk, T *x, const T *g, const T *c,
       a.pold = iter == 1 ? nullptr : pold;
       a.c_unit_interior = std::is_same<T, float>::value && wk.c32_face ? 1 : 0;
       a.g_uniform = std::is_same<T, float>::value ? wk.g32_uniform : 0;
+      a.box = wk.box;
+      a.box_ok = box_ok(wk);
       NB_TRY(launch_ax<T>(op, 1, a, s));
       k_gs_fin<T><<<wk.grid_gs, 256, 0, s>>>(w, p, c, op.bnd_off, op.bnd_idx,
                                              op.nbg, wk.partial_gs, wk.partial_ax,
-                                             op.nelt, wk.counters + 0, wk.sc);
+                                             op.nelt, wk.counters + 0, wk.sc, wk.box,
+                                             box_ok(wk));
       NB_CUDA(cudaGetLastError());
     } else {
       if (iter == 1)
@@ -847,12 +995,14 @@ int time_cg_kernels_t(Operator &op, CgWork &wk, T *x, const T *f, const T *g,
     a.D = D;
     a.sc = wk.sc;
     a.partial = wk.partial_ax;
+    a.box = wk.box;
+    a.box_ok = box_ok(wk);
     NB_CUDA(cudaEventRecord(ev[0], s));
     NB_TRY(launch_ax<T>(op, 1, a, s));
     NB_CUDA(cudaEventRecord(ev[1], s));
     k_gs_fin<T><<<wk.grid_gs, 256, 0, s>>>(w, pc, c, op.bnd_off, op.bnd_idx, op.nbg,
                                            wk.partial_gs, wk.partial_ax, op.nelt,
-                                           wk.counters + 0, wk.sc);
+                                           wk.counters + 0, wk.sc, wk.box, box_ok(wk));
     NB_CUDA(cudaEventRecord(ev[2], s));
     if (!PAIRED)
       update_launch<T, 0>(op, wk, x, r, pc, w, c, nullptr, it + 2, 1, nullptr, nullptr, s);
@@ -879,21 +1029,11 @@ template int time_cg_kernels_t<float>(Operator &, CgWork &, float *, const float
                                       const float *, const float *, float *, float *,
                                       float *, int, double *, cudaStream_t);
 
-int launch_gs_fin(const Operator &op, CgWork &wk, double *w, const double *p,
-                  const double *c, cudaStream_t s) {
-  k_gs_fin<double><<<wk.grid_gs, 256, 0, s>>>(w, p, c, op.bnd_off, op.bnd_idx,
-                                              op.nbg, wk.partial_gs, wk.partial_ax,
-                                              op.nelt, wk.counters + 0, wk.sc);
-  NB_CUDA(cudaGetLastError());
-  return NB_OK;
-}
-
-int launch_cg_update(const Operator &op, CgWork &wk, double *x, double *r,
-                     const double *p, const double *w, const double *c,
-                     int iter, cudaStream_t s) {
-  k_cg_update<double><<<wk.grid_up, 256, 0, s>>>(x, r, p, w, c, op.n, wk.partial_up,
-                                                 wk.counters + 1, wk.sc, nullptr,
-                                                 iter, 1);
+// w of the last iteration finished at the boundary points, for the caller
+template <typename T>
+static int finish_w(const Operator &op, const CgWork &wk, T *w, const T *p, cudaStream_t s) {
+  if (wk.box.nx == 0) return NB_OK;
+  k_box_finish<T><<<wk.grid_gs, 256, 0, s>>>(w, p, op.bnd_off, op.bnd_idx, op.nbg, box_ok(wk));
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
@@ -902,7 +1042,7 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
               const double *g, const double *c, double *r, double *w,
               double *p, double *z, int niter, Precond *M, bool force_unfused,
               cudaStream_t s) {
-  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, true, niter, s));
+  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, !M && !force_unfused, niter, s));
   // the second direction buffer of the paired x update (fused, no
   // preconditioner, at least one pair)
   double *p_alt = nullptr;
@@ -912,6 +1052,8 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
   }
   NB_TRY(cg_steps_t<double>(op, wk, x, g, c, r, w, p, z, 1, niter, niter, M,
                             force_unfused, s, p_alt));
+  if (niter > 0)
+    NB_TRY(finish_w<double>(op, wk, w, p_alt && niter % 2 == 0 ? p_alt : p, s));
   // the last direction is the caller's p (cg.f's p on return)
   if (p_alt && niter % 2 == 0)
     NB_CUDA(cudaMemcpyAsync(p, p_alt, op.n * sizeof(double), cudaMemcpyDeviceToDevice, s));
@@ -919,8 +1061,8 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
 }
 
 int cg_begin(Operator &op, CgWork &wk, double *x, const double *f,
-             const double *c, double *r, int niter, cudaStream_t s) {
-  return cg_begin_t<double>(op, wk, x, f, c, r, true, niter, s);
+             const double *c, double *r, int niter, bool precond, cudaStream_t s) {
+  return cg_begin_t<double>(op, wk, x, f, c, r, !precond, niter, s);
 }
 
 int cg_steps(Operator &op, CgWork &wk, double *x, const double *g,
@@ -938,10 +1080,12 @@ int cg_steps_pc(Operator &op, CgWork &wk, double *x, const double *g,
 
 int cg_device_f32(Operator &op, CgWork &wk, float *x, const float *f,
                   const float *g, const float *c, float *r, float *w, float *p,
-                  int niter, cudaStream_t s, float *p_alt) {
-  NB_TRY(cg_begin_t<float>(op, wk, x, f, c, r, true, niter, s));
-  return cg_steps_t<float>(op, wk, x, g, c, r, w, p, r, 1, niter, niter,
-                           nullptr, false, s, p_alt);
+                  int niter, cudaStream_t s, float *p_alt, bool want_w) {
+  NB_TRY(cg_begin_t<float>(op, wk, x, f, c, r, !wk.tc_inner, niter, s));
+  NB_TRY(cg_steps_t<float>(op, wk, x, g, c, r, w, p, r, 1, niter, niter,
+                           nullptr, false, s, p_alt));
+  if (!want_w || niter < 1) return NB_OK;
+  return finish_w<float>(op, wk, w, p_alt && niter % 2 == 0 ? p_alt : p, s);
 }
 
 }  // namespace nb

@@ -59,6 +59,14 @@ struct Operator {
   unsigned *bnd_idx = nullptr;      // with mask flags in bit 31
   cudaStream_t stream = nullptr;
   bool brick = false;               // box in the brick element order (lglel(e) = e)
+  bool box_groups = false;           // the boundary groups are a brick box's copies
+  unsigned char *d_mask0 = nullptr;  // a box's mask list as flags of element 0's points
+  bool mask0_ok = false;             //   (no other element masked)
+  unsigned *d_bnd_pts = nullptr;     // BoxMesh::bnd
+  int n_bnd_pts = 0;
+  // the box for the assembled update (nb_kernels.cuh); nx = 0 where the mesh
+  // or its mask is not of that form
+  BoxMesh box_mesh() const;
 
   ~Operator();
 };
@@ -89,6 +97,9 @@ struct CgWork {
   // multiplicity (c_closed_form): each element's face bits; the fused
   // iteration then forms c instead of reading it (same values)
   const unsigned char *c32_face = nullptr;
+  // the solve begun takes the assembled update where its check on the device
+  // holds (sc->box_ok); nx = 0: the general iteration
+  BoxMesh box{};
   // the FP64 CG's second direction buffer (paired x update)
   double *palt = nullptr;
   long palt_n = 0;
@@ -203,8 +214,9 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
               cudaStream_t s);
 // The same iteration split in two: the set-up of cg.f:36-42, then
 // iterations it0..it1 (identity preconditioner), scalars kept on the device.
+// precond: the iterations will be preconditioned (cg_steps_pc).
 int cg_begin(Operator &op, CgWork &wk, double *x, const double *f,
-             const double *c, double *r, int niter, cudaStream_t s);
+             const double *c, double *r, int niter, bool precond, cudaStream_t s);
 int cg_steps(Operator &op, CgWork &wk, double *x, const double *g,
              const double *c, double *r, double *w, double *p, int it0,
              int it1, cudaStream_t s);
@@ -221,12 +233,6 @@ template <typename T>
 int time_cg_kernels_t(Operator &op, CgWork &wk, T *x, const T *f, const T *g,
                       const T *c, T *r, T *w, T *p, int reps, double *ms3,
                       cudaStream_t s);
-// the second and third kernels of a fused FP64 iteration, for timing
-int launch_gs_fin(const Operator &op, CgWork &wk, double *w, const double *p,
-                  const double *c, cudaStream_t s);
-int launch_cg_update(const Operator &op, CgWork &wk, double *x, double *r,
-                     const double *p, const double *w, const double *c,
-                     int iter, cudaStream_t s);
 // iterations it0..it1 with preconditioner M (z = M^-1 r), scalars on device
 int cg_steps_pc(Operator &op, CgWork &wk, double *x, const double *g,
                 const double *c, double *r, double *w, double *p, double *z,
@@ -249,8 +255,9 @@ int c_closed_form(const Operator &op, const float *c32, unsigned char *cface, in
 // With p_alt (a second n-point direction buffer) the fused iterations
 // alternate their directions between p and p_alt and update x once per two
 // iterations (bitwise the same iterates, 8 fewer bytes a point per pair).
+// want_w: the caller reads w (A p of the last iteration) afterwards.
 int cg_device_f32(Operator &op, CgWork &wk, float *x, const float *f,
                   const float *g, const float *c, float *r, float *w, float *p,
-                  int niter, cudaStream_t s, float *p_alt = nullptr);
+                  int niter, cudaStream_t s, float *p_alt = nullptr, bool want_w = true);
 
 }  // namespace nb

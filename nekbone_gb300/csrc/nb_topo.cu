@@ -270,6 +270,7 @@ int box_topology_device(Operator *op, cudaStream_t s) {
   op->fused_ok = true;
   op->mask_built = op->mask_mode == 1;
   op->brick = true;
+  op->box_groups = true;
   return NB_OK;
 }
 
