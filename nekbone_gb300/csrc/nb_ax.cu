@@ -25,9 +25,12 @@ int launch_ax<double>(const Operator &op, int mode, AxArgs<double> a, cudaStream
   a.err = device_error_word();
   a.wait_test = wait_test_mode();
   if (op.order == 2 && op.fx_ok) {  // fixed point on the integer pipes
-    NB_TRY(metric_fx_prepare(op, a.g, s));
+    NB_TRY(metric_fx_prepare(op, a.g, op.dD, s));
     a.gfx = op.gfx;
     a.gexp = op.gexp;
+    a.sep = op.sep_on ? op.sep : nullptr;
+    if (mode == 0 && a.sep)
+      return fail(NB_ERR_STATE, "ax: a plain apply inside a solve on the separable metric");
     if (mode == 0) return launch_ax_fx_m0(op, a, s);
     if (mode == 1) return launch_ax_fx_m1(op, a, s);
     return launch_ax_fx_m2(op, a, s);

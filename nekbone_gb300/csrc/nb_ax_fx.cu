@@ -55,10 +55,12 @@ int64_t scaled_sum(const double *x, int nx, int sh) {
 
 // one block per element: the element's largest exponent over its 6 lx1^3
 // metric values, then each value as balanced halves of g 2^(1082 - emax)
+// (nothing where the separable form holds)
 __global__ void __launch_bounds__(256)
     k_metric_fx(const double *__restrict__ g, int2 *__restrict__ gfx, int *__restrict__ gexp,
-                int blk) {
+                int blk, const fx::SepTables *sep) {
   __shared__ int wmax[8];
+  if (sep && sep->ok) return;
   const int t = threadIdx.x;
   const size_t base = size_t(blockIdx.x) * blk;
   int em = 0;
@@ -73,6 +75,139 @@ __global__ void __launch_bounds__(256)
     gfx[base + q] = make_int2(s.lo, s.hi);
   }
   if (t == 0) gexp[blockIdx.x] = em;
+}
+
+// ------------------------------------------------------ double-double --
+struct DD {
+  double h, l;
+};
+__device__ __forceinline__ DD dd_sum(double a, double b) {  // exact (Knuth's two-sum)
+  const double s = __dadd_rn(a, b), bb = __dadd_rn(s, -a);
+  return {s, __dadd_rn(__dadd_rn(a, -__dadd_rn(s, -bb)), __dadd_rn(b, -bb))};
+}
+__device__ __forceinline__ DD dd_add(DD a, DD b) {
+  const DD s = dd_sum(a.h, b.h);
+  return dd_sum(s.h, __dadd_rn(s.l, __dadd_rn(a.l, b.l)));
+}
+
+// K and its fixed-point tables from D and element 0's v, by one block:
+// K(i,m) in double-double for the upper rows i < h, then E and O, each the
+// nearest integer of the value times 2^fc.  Like the even-odd tables of the
+// general form it takes D's upper rows and their mirror images; b is made
+// symmetric (K then is).  False where a sum of the operator's accumulators
+// (Acc, and the three directions) could leave 64 bits.
+__device__ bool sep_tables(const double *__restrict__ D, int lx, fx::SepTables *sep) {
+  __shared__ DD K[128];
+  __shared__ double bs[16];
+  __shared__ int emax[8];
+  const int t = threadIdx.x, h = lx / 2, n1 = lx - 1, nk = h * lx;
+  if (t < lx) {
+    const int at = lx * h + lx * lx * h;
+    bs[t] = 0.5 * (sep->v[t + at] + sep->v[n1 - t + at]);
+  }
+  __syncthreads();
+  int em = 0;
+  if (t < nk) {
+    const int i = t / lx, m = t % lx;
+    auto Du = [&](int r, int c) { return r < h ? D[r + c * lx] : -D[n1 - r + (n1 - c) * lx]; };
+    DD k = {0.0, 0.0};
+    for (int q = 0; q < lx; ++q) {
+      const double a = Du(q, i), b = Du(q, m), w = bs[q];
+      const double p = __dmul_rn(a, b), pe = __fma_rn(a, b, -p);  // a b = p + pe
+      const double r = __dmul_rn(p, w), re = __fma_rn(pe, w, __fma_rn(p, w, -r));
+      const DD x = dd_sum(k.h, r);
+      k = {x.h, __dadd_rn(k.l, __dadd_rn(x.l, re))};
+    }
+    const double w = bs[i], q = __ddiv_rn(k.h, w), r = __fma_rn(-q, w, k.h);  // r exact
+    k = dd_sum(q, __ddiv_rn(__dadd_rn(r, k.l), w));
+    K[t] = k;
+  }
+  __syncthreads();
+  // value t of the tables, and the largest exponent among them
+  DD p = {0.0, 0.0};
+  if (t < 2 * h * h) {
+    const int a = (t % (h * h)) / h, c = t % h;
+    const double s = t < h * h ? 0.5 : -0.5;  // E, O
+    const DD x = K[a * lx + c], y = K[a * lx + n1 - c];
+    p = dd_add(DD{0.5 * x.h, 0.5 * x.l}, DD{s * y.h, s * y.l});
+    em = fx::bexp(p.h);
+  }
+  em = int(__reduce_max_sync(0xFFFFFFFFu, unsigned(em)));
+  if ((t & 31) == 0) emax[t >> 5] = em;
+  __syncthreads();
+  for (int q = 0; q < 8; ++q) em = max(em, emax[q]);
+  const int fc = 61 - (em - 1022);  // every value below 2^(em - 1022)
+  bool good = em > 1 && em < 2046;
+  if (good && t < 2 * h * h) {
+    // the high part times 2^fc has a fraction of at most 52 bits: both exact
+    const double hs = scalbn(p.h, fc), hi = rint(hs);
+    const long long C = (long long)hi + __double2ll_rn((hs - hi) + scalbn(p.l, fc));
+    const fx::Sp sp = fx::split(C);
+    sep->tab[t] = make_int2(sp.hi, sp.lo);
+    good = C <= (1ll << 61) && C >= -(1ll << 61);
+  }
+  __syncthreads();
+  if (good && t < h) {  // the rows' sums
+    double xe = 0.0, xo = 0.0, hm = 0.0;
+    for (int c = 0; c < h; ++c) {
+      const int2 e = sep->tab[t * h + c], o = sep->tab[h * h + t * h + c];
+      const double ae = fabs(double(e.x)) + 1.0, ao = fabs(double(o.x)) + 1.0;
+      // x + x2 of a sum, in units of 2^31: |hi| 2^31 + |lo| 2^29 a term
+      xe += ae + 0.25 * fabs(double(e.y));
+      xo += ao + 0.25 * fabs(double(o.y));
+      hm += fmax(ae, ao);
+    }
+    // the output: three directions of at most sum max(|E|, |O|) times 2^61, in
+    // units of 2^64
+    good = xe < 4.29e9 && xo < 4.29e9 && 3.0 * hm < 1.7e10;
+  }
+  if (t == 0) sep->fc = fc;
+  return good;
+}
+
+// Whether g has the separable form (SepTables): sep->ok, set before, is
+// cleared where it has not, and a block returns at once when it finds it
+// cleared.  Block 0 looks at element 0's product form and makes the tables
+// meanwhile; every block compares its elements with element 0, bitwise.
+// HBM-bound: g read once (48 B a point, 0.39 ms at 32^3, lx1 = 12) where the
+// form holds, next to nothing where it does not.
+__global__ void __launch_bounds__(256)
+    k_sep_check(const double *__restrict__ g, const double *__restrict__ D, int lx, int nelt,
+                fx::SepTables *sep) {
+  const int l3 = lx * lx * lx, t = threadIdx.x;
+  const unsigned long long *g0 = reinterpret_cast<const unsigned long long *>(g);
+  __shared__ int on;
+  for (int e = blockIdx.x; e < nelt; e += gridDim.x) {
+    if (t == 0) on = *reinterpret_cast<volatile int *>(&sep->ok);
+    __syncthreads();
+    if (!on) return;
+    bool ok = true;
+    const unsigned long long *ge = g0 + size_t(e) * 6 * l3;
+    for (int l = t; l < l3; l += blockDim.x) {
+      const unsigned long long v = g0[6 * l];
+      const unsigned long long *q = ge + 6 * l;
+      ok &= q[0] == v && q[3] == v && q[5] == v && ((q[1] | q[2] | q[4]) << 1) == 0;
+    }
+    if (e == 0 && __syncthreads_and(ok)) {
+      const int m = lx / 2, L2 = lx * lx;
+      auto line = [&](int i) { return g[6 * (i + lx * m + L2 * m)]; };
+      const double gm = line(m);
+      for (int l = t; l < l3; l += blockDim.x) {
+        const double v = g[6 * l];
+        const double a = line(l % lx), b = line((l / lx) % lx), c = line(l / L2);
+        const double l1 = v * gm * gm, l2 = a * b * c;
+        // (2e-15: up to eight roundings on each side), b symmetric likewise
+        ok &= v > 1e-60 && v < 1e60 && fabs(l1 - l2) <= 2e-15 * l2;
+        ok &= fabs(a - line(lx - 1 - l % lx)) <= 2e-15 * a;
+        sep->v[l] = v;
+      }
+      if (__syncthreads_and(ok)) ok = sep_tables(D, lx, sep);
+    }
+    if (!__syncthreads_and(ok)) {
+      if (t == 0) atomicExch(&sep->ok, 0);
+      return;
+    }
+  }
 }
 
 }  // namespace
@@ -153,23 +288,36 @@ bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
   return ok;
 }
 
-void metric_fx_invalidate(const Operator &op) { op.gfx_src = nullptr; }
+void metric_fx_invalidate(const Operator &op, bool solve) {
+  op.gfx_src = nullptr;
+  op.metric_solve = solve;
+}
 
-int metric_fx_prepare(const Operator &op, const double *g, cudaStream_t s) {
+int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s) {
   if (op.gfx_src == g && op.gfx) return NB_OK;
   const long nv = 6 * op.n;
   if (op.gfx_cap < nv) {
     if (op.gfx) cudaFree(op.gfx);
-    if (op.gexp) cudaFree(op.gexp);
+    if (op.sep) cudaFree(op.sep);
+    op.sep = nullptr;
     op.gfx = nullptr;
     op.gexp = nullptr;
     op.gfx_cap = 0;
     NB_CUDA(cudaMalloc(&op.gfx, size_t(nv) * sizeof(int2)));
-    NB_CUDA(cudaMalloc(&op.gexp, size_t(op.nelt) * sizeof(int)));
+    // the separable form's tables and the exponents: one allocation
+    NB_CUDA(cudaMalloc(&op.sep, sizeof(fx::SepTables) + size_t(op.nelt) * sizeof(int)));
+    op.gexp = reinterpret_cast<int *>(op.sep + 1);
     op.gfx_cap = nv;
   }
   const int blk = 6 * op.lx * op.lx * op.lx;
-  k_metric_fx<<<op.nelt, 256, 0, s>>>(g, op.gfx, op.gexp, blk);
+  // the separable form's check pays from the second apply on
+  const bool sep = op.metric_solve && op.lx % 2 == 0;
+  op.sep_on = sep;
+  if (sep) {
+    NB_CUDA(cudaMemsetAsync(&op.sep->ok, 1, sizeof(int), s));
+    k_sep_check<<<std::min(op.nelt, 152 * 8), 256, 0, s>>>(g, D, op.lx, op.nelt, op.sep);
+  }
+  k_metric_fx<<<op.nelt, 256, 0, s>>>(g, op.gfx, op.gexp, blk, sep ? op.sep : nullptr);
   NB_CUDA(cudaGetLastError());
   op.gfx_src = g;
   return NB_OK;

@@ -223,8 +223,9 @@ __device__ __forceinline__ double to_double_cvt(i64 W, int s) {
   const i64 b = __double_as_longlong(d);
   const int e = int((b >> 52) & 0x7FF);
   const int e2 = e + s;
-  if (d != 0.0 && e2 >= 1 && e2 <= 2046) return __longlong_as_double(b + (i64(s) << 52));
-  return d == 0.0 ? 0.0 : to_double(W, s);
+  // (zero is looked for in W: a comparison of d is one more FP64 operation)
+  if (W != 0 && e2 >= 1 && e2 <= 2046) return __longlong_as_double(b + (i64(s) << 52));
+  return W == 0 ? 0.0 : to_double(W, s);
 }
 // x * 2^(1075 - emax + up) rounded to the nearest integer, ties to even
 // (to_fixed rounds them away from zero), by an exact FP64 scaling and the
@@ -235,6 +236,17 @@ __device__ __forceinline__ i64 to_fixed_cvt(double x, int emax, int up) {
   if (k > 1023 || k < -1022) return to_fixed(x, emax, up);  // 2^k not a normal double
   const double sc = __longlong_as_double(i64(k + 1023) << 52);
   return __double2ll_rn(x * sc);
+}
+// x * 2^(1082 - emax) rounded to nearest (halves away from zero), |result| <=
+// 2^60, for x whose biased exponent is <= emax, on the integer pipes
+__device__ __forceinline__ i64 to_fixed60(double x, int emax) {
+  if (emax < 128) return to_fixed(x, emax, 7);  // (near the subnormals; uniform)
+  const u64 b = u64(__double_as_longlong(x));
+  const int e = int((b >> 52) & 0x7FFu);
+  const int r = min(emax - e, 63);  // a zero (e = 0) shifts out
+  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 8;
+  const i64 v = i64(((m >> r) + 1ull) >> 1), s = i64(b) >> 63;
+  return (v ^ s) - s;
 }
 // ----------------------------------------------------- block reductions --
 // lanes of warp w of an nt-thread block
@@ -277,9 +289,30 @@ struct FxCoef {
 template <int LX>
 constexpr int fx_bits() { return FxCoef<LX>::FULL ? 61 : 59; }
 
+// ------------------------------------------------------ separable metric --
+// A box of equal cubes (setup_g, prox_setup.f:27-52) has the same block in
+// every element, G1 = G4 = G6 = v(i,j,k) and G2 = G3 = G5 = 0, with v a
+// product of one-dimensional weights, v = s b_i b_j b_k.  There
+//   D^T diag(v) D  along i  =  v K along i,   K(i,m) = sum_q D(q,i) b_q/b_i D(q,m),
+// so w_L = v (K u along i + along j + along k): three contractions instead of
+// six, no metric step and no metric read but one shared block.  k_sep_check
+// establishes the form on the device, once per solve, from g itself (every
+// element bitwise, the product to the rounding of its factors), and makes K in
+// double-double.  ok = 0: the general form.
+struct SepTables {
+  int ok, fc;        // fc: fractional bits of the tables
+  int pad[2];
+  // (hi, lo) of E, then of O, h x h each (row a), |coefficient| <= 2^61; K is
+  // centrosymmetric: y(a) = E ve + O vo, y(n-1-a) = E ve - O vo
+  int2 tab[2 * 64];
+  double v[4096];
+};
+
 template <int LX>
 struct FxShared {
   static constexpr int N = (LX * LX + 1) * LX;
+  static constexpr int NT = FxCoef<LX>::FULL ? 2 : 2 * (LX / 2) * (LX / 2);
+  alignas(16) int2 tab[NT];  // SepTables' tables
   i64 A[N];
   i64 C[N];
   i64 D[N];
@@ -349,6 +382,31 @@ __device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int 
   }
 }
 
+// y = K v of one line, |v| < 2^60 (SepTables)
+template <int LX, typename Put>
+__device__ __forceinline__ void fx_line_sep(const i64 *v, const int2 *tab, Put put) {
+  constexpr int H = LX / 2;
+  Sp ve[H], vo[H];
+#pragma unroll
+  for (int m = 0; m < H; ++m) {
+    ve[m] = split(v[m] + v[LX - 1 - m]);
+    vo[m] = split(v[m] - v[LX - 1 - m]);
+  }
+#pragma unroll 1
+  for (int a = 0; a < H; ++a) {
+    Acc<0> e, o;
+#pragma unroll
+    for (int m = 0; m < H; ++m) {
+      const int2 ce = tab[a * H + m], co = tab[H * H + a * H + m];
+      e.mac(Sp{ce.y, ce.x}, ve[m]);
+      o.mac(Sp{co.y, co.x}, vo[m]);
+    }
+    const i64 ye = e.result(), yo = o.result();
+    put(a, ye + yo);
+    put(LX - 1 - a, ye - yo);
+  }
+}
+
 // OR of the magnitudes of a thread's values, combined over the block after
 // the next __syncthreads (fx_or_read): its top bit is the largest's
 __device__ __forceinline__ void fx_or_post(u64 v, unsigned *orl, unsigned *orh, int t, int nt) {
@@ -372,6 +430,170 @@ __device__ __forceinline__ int fx_or_shift(const unsigned *orl, const unsigned *
 // exact negative power of two, which the bounds leave room for)
 __device__ __forceinline__ u64 mag(i64 v) { return u64(v ^ (v >> 63)); }
 
+// The end of element e at the thread's column (i, j): w_L of its point k is
+// wloc(k) (bad: the element has a value that is not finite, which has no
+// fixed-point form); the CG epilogue as k_ax_eo's.  Points k0 .. k0 + NK - 1,
+// the thread's part of the reduction returned. 
+template <int LX, int MODE, int NK, bool WHOLE, typename W>
+__device__ __forceinline__ double ax_fx_finish(const AxArgs<double> &a, int e, int t, int k0,
+                                               bool bad, unsigned nbr, W wloc) {
+  constexpr int L2 = LX * LX, L3 = LX * LX * LX;
+  const int i = t % LX, j = t / LX;
+  const size_t base = size_t(e) * L3;
+  // p (written above by this thread, so in cache), c and f are read again
+  // here rather than held in registers through the contractions
+  const bool col_interior = (i > 0) && (i < LX - 1) && (j > 0) && (j < LX - 1);
+  double part = 0.0;
+  double pk[NK], ck[NK], fk[NK];
+  if (WHOLE || (MODE != 0 && col_interior)) {
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {  // all loads before the first store
+      const int k = k0 + q;
+      if (k >= LX) break;
+      const size_t id = base + size_t(k) * L2 + t;
+      const bool interior = k > 0 && k < LX - 1;
+      if (WHOLE || interior) pk[q] = a.p[id];
+      if (!WHOLE && interior) ck[q] = __ldg(a.c + id);
+      if (MODE == 2 && interior) fk[q] = __ldg(a.f + id);
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < NK; ++q) {
+    const int k = k0 + q;
+    if (k >= LX) break;
+    double wl = wloc(k);
+    if (bad) wl = __longlong_as_double(0x7FF8000000000000ll);
+    const size_t id = base + size_t(k) * L2 + t;
+    const bool interior = col_interior && (k > 0) && (k < LX - 1);
+    if (WHOLE) {
+      wl = fma_rn(box_tenth<double>(box_ext<LX>(i, j, k) & nbr), pk[q], wl);
+      part = fma_rn(wl, pk[q], part);
+      a.w[id] = wl;
+    } else if (MODE == 1) {
+      if (interior) {
+        wl = fma_rn(0.1, pk[q], wl);
+        part = fma_rn(mul_rn(wl, ck[q]), pk[q], part);
+      }
+      a.w[id] = wl;
+    } else if (MODE == 2) {
+      if (interior) {
+        const double rv = fk[q] - fma_rn(0.1, pk[q], wl);
+        a.r[id] = rv;
+        part = fma_rn(mul_rn(rv, ck[q]), rv, part);
+      } else {
+        a.w[id] = wl;
+      }
+    } else {
+      a.w[id] = wl;
+    }
+  }
+  return part;
+}
+
+// ----------------------------------------------- separable-metric operator --
+// The operator where SepTables' form holds (MODE 1 and 2 as ax_fx_body).  Two
+// of the shared arrays: the element in fixed point (A), and the sum of the
+// three directions' results (C), each direction's lines added by the threads
+// that own them.  About 300 instructions a point at half an issue a cycle and
+// five FP64 operations (58 % of that pipe): 0.86 ms at 32^3, lx1 = 12, against
+// 1.53 for the general form.  Measured and left out: the result's conversion
+// and product on the integer pipes (40 instructions for two FP64 operations,
+// 0.88 to 0.95 ms); two elements a CTA (0.88); a kernel of its own with six
+// CTAs per SM (0.81 to 0.86, but 3 to 6 us a launch on small meshes, since
+// the device decides which of the two runs).
+template <int LX, int MODE>
+__device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX> &sm, bool whole,
+                                            unsigned nbr, int fc) {
+  constexpr int L2 = LX * LX, L3 = LX * LX * LX, NT = FxShared<LX>::NT;
+  const int t = threadIdx.x + LX * threadIdx.y;
+  const int i = threadIdx.x, j = threadIdx.y;  // own column (i,j)
+  const int e = blockIdx.x;
+  const size_t base = size_t(e) * L3;
+  if (t < NT) sm.tab[t] = a.sep->tab[t];
+
+  int em = 0;
+  {
+    double uk[LX];
+    const double beta = (MODE == 1 && !a.first) ? a.sc->beta : 0.0;
+    constexpr int HB = LX / 2;
+#pragma unroll
+    for (int k0 = 0; k0 < LX; k0 += HB) {  // two halves: fewer values held at once
+      double pold[HB];
+#pragma unroll
+      for (int q = 0; q < HB; ++q) {  // all loads before the first store
+        const size_t id = base + size_t(k0 + q) * L2 + t;
+        if (MODE == 1) {
+          uk[k0 + q] = a.u[id];
+          pold[q] = a.first ? 0.0 : a.pold[id];
+        } else {
+          uk[k0 + q] = a.p[id];
+          pold[q] = a.e ? double(a.e[id]) : 0.0;
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < HB; ++q) {
+        const int k = k0 + q;
+        const size_t id = base + size_t(k) * L2 + t;
+        if (MODE == 1) {
+          if (!a.first) uk[k] = fma_rn(beta, pold[q], uk[k]);  // add2s1, math.f:534
+          a.p[id] = uk[k];
+        } else if (a.e) {
+          uk[k] = fma_rn(a.scale, pold[q], uk[k]);
+          a.p[id] = uk[k];
+        }
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < LX; ++k) em = max(em, bexp(uk[k]));
+    const int w = t >> 5;
+    const int r = __reduce_max_sync(warp_mask(L2, w), unsigned(em));
+    if ((t & 31) == 0) sm.emax[w] = r;
+    __syncthreads();
+    em = 0;
+    for (int q = 0; q < (L2 + 31) / 32; ++q) em = max(em, sm.emax[q]);
+    // (on the integer pipes: this form is held by the FP64 one)
+#pragma unroll
+    for (int k = 0; k < LX; ++k) sm.A[fx_at<LX>(i, j, k)] = to_fixed60(uk[k], em);
+  }
+  __syncthreads();
+
+  // K along j, then i, then k (the own column); run-time strides keep one copy
+  // of the line code
+#pragma unroll 1
+  for (int d = 0; d < 3; ++d) {
+    if (d) __syncthreads();
+    const int b0 = d == 0 ? fx_at<LX>(i, 0, j) : d == 1 ? fx_at<LX>(0, j, i) : fx_at<LX>(i, j, 0);
+    const int st = d == 0 ? LX : d == 1 ? 1 : (LX * LX + 1);
+    i64 v[LX];
+#pragma unroll
+    for (int m = 0; m < LX; ++m) v[m] = sm.A[b0 + m * st];
+    fx_line_sep<LX>(v, sm.tab, [&](int m, i64 y) {
+      i64 *o = sm.C + b0 + m * st;
+      *o = d ? *o + y : y;
+    });
+  }
+
+  const int sY = em - 1075 - (60 - 53) + 64 - fc;
+  const bool bad = em == 0x7FF;
+  constexpr int NK = LX / 2;
+  double part = 0.0;
+#pragma unroll
+  for (int k0 = 0; k0 < LX; k0 += NK) {
+    double vk[NK];
+#pragma unroll
+    for (int q = 0; q < NK; ++q) vk[q] = __ldg(a.sep->v + (k0 + q) * L2 + t);
+    auto wloc = [&](int k) {
+      return mul_rn(to_double_cvt(sm.C[fx_at<LX>(i, j, k)], sY), vk[k - k0]);
+    };
+    if (MODE == 1 && whole)
+      part += ax_fx_finish<LX, MODE, NK, MODE == 1>(a, e, t, k0, bad, nbr, wloc);
+    else
+      part += ax_fx_finish<LX, MODE, NK, false>(a, e, t, k0, bad, nbr, wloc);
+  }
+  const double s = block_sum<double>(part, sm.red);
+  if (t == 0) a.partial[e] = s;
+}
+
 // MODE 0 / 1 / 2 as k_ax_eo (AxArgs); a.gfx / a.gexp hold the metric in
 // fixed point (metric_fx_prepare).
 template <int LX, int MODE>
@@ -385,6 +607,15 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   const size_t base = size_t(e) * L3;
   const int fc = cf.fc;
   if (a.act && !a.act[size_t(a.el_prob[e]) * a.act_stride]) return;  // the whole CTA
+  const bool whole = MODE == 1 && box_flag(a.box_ok);  // pap formed here (BoxMesh)
+  const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
+  if constexpr (MODE != 0 && !FxCoef<LX>::FULL) {
+    const int2 sep = a.sep ? *reinterpret_cast<const int2 *>(a.sep) : make_int2(0, 0);
+    if (sep.x) {
+      ax_sep_body<LX, MODE>(a, sm, whole, nbr, sep.y);
+      return;
+    }
+  }
 
   // direction update (MODE 1) / correction (MODE 2), in FP64, then the
   // element's exponent and its fixed-point block
@@ -511,55 +742,17 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   }
   __syncthreads();
 
-  // w_L = tr + ts + tt in FP64; the CG epilogue as k_ax_eo's.  p (written
-  // above by this thread, so in cache), c and f are read again here rather
-  // than held in registers through the contractions.
-  const bool whole = MODE == 1 && box_flag(a.box_ok);  // pap formed here (BoxMesh)
-  const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
-  const bool col_interior = (i > 0) && (i < LX - 1) && (j > 0) && (j < LX - 1);
-  // an element with a value that is not finite has no fixed-point form
-  const bool bad = em == 0x7FF || eg == 0x7FF;
-  double part = 0.0;
-  double pk[LX], ck[LX], fk[LX];
-  if (MODE != 0 && (col_interior || whole)) {
-#pragma unroll
-    for (int k = 0; k < LX; ++k) {  // all loads before the first store
-      const size_t id = base + size_t(k) * L2 + t;
-      const bool interior = col_interior && k > 0 && k < LX - 1;
-      if (interior || whole) pk[k] = a.p[id];
-      if (interior && !whole) ck[k] = __ldg(a.c + id);
-      if (MODE == 2 && interior) fk[k] = __ldg(a.f + id);
-    }
-  }
-#pragma unroll
-  for (int k = 0; k < LX; ++k) {
+  // w_L = tr + ts + tt in FP64
+  auto wloc = [&](int k) {
     const int q = fx_at<LX>(i, j, k);
-    double wl = to_double_cvt(sm.A[q] + sm.C[q] + sm.D[q], sT);
-    if (bad) wl = __longlong_as_double(0x7FF8000000000000ll);
-    const size_t id = base + size_t(k) * L2 + t;
-    const bool interior = col_interior && (k > 0) && (k < LX - 1);
-    if (MODE == 1) {
-      if (whole) {
-        const double wv = fma_rn(box_tenth<double>(box_ext<LX>(i, j, k) & nbr), pk[k], wl);
-        part = fma_rn(wv, pk[k], part);
-        if (interior) wl = wv;
-      } else if (interior) {
-        wl = fma_rn(0.1, pk[k], wl);
-        part = fma_rn(mul_rn(wl, ck[k]), pk[k], part);
-      }
-      a.w[id] = wl;
-    } else if (MODE == 2) {
-      if (interior) {
-        const double rv = fk[k] - fma_rn(0.1, pk[k], wl);
-        a.r[id] = rv;
-        part = fma_rn(mul_rn(rv, ck[k]), rv, part);
-      } else {
-        a.w[id] = wl;
-      }
-    } else {
-      a.w[id] = wl;
-    }
-  }
+    return to_double_cvt(sm.A[q] + sm.C[q] + sm.D[q], sT);
+  };
+  const bool bad = em == 0x7FF || eg == 0x7FF;
+  double part;
+  if (MODE == 1 && whole)
+    part = ax_fx_finish<LX, MODE, LX, MODE == 1>(a, e, t, 0, bad, nbr, wloc);
+  else
+    part = ax_fx_finish<LX, MODE, LX, false>(a, e, t, 0, bad, nbr, wloc);
   if (MODE != 0) {
     const double s = block_sum<double>(part, sm.red);
     if (t == 0) a.partial[e] = s;
@@ -573,6 +766,7 @@ __global__ void __launch_bounds__((LX * LX + 31) / 32 * 32, (LX <= 12 ? NB_FX_MI
     k_ax_fx(AxArgs<double> a, const __grid_constant__ FxCoef<LX> cf) {
   ax_fx_body<LX, MODE>(a, cf);
 }
+
 
 template <int LX>
 constexpr size_t ax_fx_smem_bytes() {

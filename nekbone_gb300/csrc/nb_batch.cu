@@ -729,6 +729,7 @@ struct Batch {
       a.nelt = G.nel;
       a.gfx = G.fx->gfx;
       a.gexp = G.fx->gexp;
+      a.sep = G.fx->sep_on ? G.fx->sep : nullptr;
       a.el_prob = el_prob + G.el0;
       a.act = &sc[0].active;
       a.act_stride = int(sizeof(BatchScalars) / sizeof(int));
@@ -759,8 +760,8 @@ struct Batch {
   int convert_metric(cudaStream_t s) const {
     for (const auto &G : groups)
       if (G.fx && G.tune.epb64 == kFxShape) {
-        metric_fx_invalidate(*G.fx);
-        NB_TRY(metric_fx_prepare(*G.fx, g + 6 * G.pt0, s));
+        metric_fx_invalidate(*G.fx, true);
+        NB_TRY(metric_fx_prepare(*G.fx, g + 6 * G.pt0, G.D64, s));
       }
     return NB_OK;
   }
@@ -1324,8 +1325,8 @@ int nb_batch_setup(nb_batch *b, uint64_t seed) {
   // every solve converts it again)
   for (auto &G : B.groups)
     if (G.fx) {
-      metric_fx_invalidate(*G.fx);
-      NB_TRY(metric_fx_prepare(*G.fx, B.g + 6 * G.pt0, s));
+      metric_fx_invalidate(*G.fx, true);
+      NB_TRY(metric_fx_prepare(*G.fx, B.g + 6 * G.pt0, G.D64, s));
     }
   NB_CUDA(cudaStreamSynchronize(s));
   B.cf_ok = cf_h != 0;

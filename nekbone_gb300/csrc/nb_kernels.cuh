@@ -16,6 +16,10 @@
 
 namespace nb {
 
+namespace fx {
+struct SepTables;
+}
+
 // ----------------------------------------------------------- arithmetic --
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
@@ -97,12 +101,12 @@ struct CgScalars {
 // A brick box (lglel(e) = e): the copies of a point are known in closed form,
 // 2^m of them, m the number of its extreme local indices on element faces
 // with a neighbour.  There a CG iteration needs no pass that writes the
-// gather-scatter sums back: the update reads each boundary point's copies of
-// w_L itself (in jl's order, so every copy forms the same sum), and, since
-// then p is equal at all copies of a point,
-//   pap = sum_points c p (sum over copies of w_L + 0.1 p)
-//       = sum over every local point of p (w_L + 0.1 c p),
-// which the element operator sums as it makes w_L.  Measured: boundary pass
+// gather-scatter sums back.  p is equal at all copies of a point and their c
+// sum to one, so the operator writes w' = w_L + 0.1 c p at every local point,
+//   w = sum over copies of w_L + 0.1 p = sum over copies of w',
+//   pap = sum_points c p w = sum over every local point of p w',
+// it sums pap as it goes, and the update reads each boundary point's copies of
+// w' itself (in jl's order, so every copy forms the same sum).  Measured: boundary pass
 // and update at 32^3, lx1 = 12, FP64: 0.406 + 0.476 -> 0.007 + 0.533 ms; FP32
 // at 24^3: 0.115 + 0.077 -> 0.007 + 0.105 ms.
 // k_box_begin checks what that takes, once per solve: c is 2^-m bitwise at
@@ -117,6 +121,7 @@ struct BoxMesh {
   const unsigned char *mask0;  // mask of element 0's points (no other element's)
   const unsigned *bnd;         // the nbnd boundary points of an element, l | ext << 16,
   int nbnd;                    //   faces first, then edges, then corners
+  const unsigned char *ext;    // box_ext of an element's lx^3 points
 };
 // bits of the local indices that are extreme: 0/1 i = 0 / lx-1, 2/3 j, 4/5 k
 __device__ __forceinline__ unsigned box_ext(int i, int j, int k, int lx) {
@@ -177,7 +182,14 @@ __device__ __forceinline__ BoxCopies box_copies(const BoxMesh &b, int q, unsigne
   c.q0 = q - ((nb & 1u) ? c.d0 : 0) - ((nb & 4u) ? c.d1 : 0) - ((nb & 16u) ? c.d2 : 0);
   return c;
 }
-// Sum of w over the copies, left to right in ascending order (jl's:
+// With element 0's own mask a masked copy has p = 0 (c copies[q0] masked): its
+// part of 0.1 p, 0.1 c p, is missing from the sum over the copies.
+template <typename T>
+__device__ __forceinline__ T box_missing(const BoxMesh &b, const BoxCopies &c, unsigned nb, T pv) {
+  const bool is = !b.full_mask && c.q0 < b.lx * b.lx * b.lx && b.mask0[c.q0];
+  return is ? mul_rn(box_tenth<T>(nb), pv) : T(0);
+}
+// Sum of w' over the copies, left to right in ascending order (jl's:
 // gather_T_add, jl/gs_local.c:60-75).
 template <typename T>
 __device__ __forceinline__ T box_sum(const T *__restrict__ w, const BoxCopies &c) {
@@ -235,6 +247,7 @@ struct AxArgs {
   int wait_test;     // timeout self-test of the bulk-copy wait (block_copy_begin)
   const int2 *gfx;   // fixed-point FP64 operator: the metric in fixed point
   const int *gexp;   //   and each element's exponent (metric_fx_prepare)
+  const fx::SepTables *sep;  // and its separable form, where sep->ok (nb_ax_fx.cuh)
   const int *el_prob;  // fixed-point operator in a batched solve: element e is
   const int *act;      //   skipped when act[el_prob[e] * act_stride] is 0 (its
   int act_stride;      //   problem is no longer active); null for one mesh
@@ -500,14 +513,14 @@ __device__ __forceinline__ void box_alpha(const T *w, const T *p, double *partia
     const unsigned nbr = box_neighbours(box, 0);
     double d = 0.0;
     for (int l = threadIdx.x; l < l3; l += blockDim.x) {
-      const unsigned cp = box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx) & nbr;
+      const unsigned cp = __ldg(box.ext + l) & nbr;
       if (!cp || !box.mask0[l]) continue;
       const BoxCopies c = box_copies(box, l, cp);
       const double t = double(box_sum(w, c)), cm = box_mult<double>(cp);
       const double pv = double(p[c.q0 + c.d0 + c.d1 + c.d2]);
       const double others = double((1 << __popc(cp)) - 1);
-      // all but element 0's copy: c p (t + 0.1 p) instead of p (w_L + 0.1 c p)
-      d += others * cm * pv * t - pv * (t - double(w[l]));
+      // all but element 0's copy: c p w instead of p w'
+      d += others * cm * pv * (t + 0.1 * cm * pv) - pv * (t - double(w[l]));
     }
     __syncthreads();
     pap += block_sum<double>(d, red);
@@ -819,32 +832,33 @@ __device__ __forceinline__ float box_scale(float r, int m) {
 }
 
 // k_cg_update with the sums over copies and the mask taken here (BoxMesh).
-// A block takes an element at a time: first its boundary points, w = sum of
-// w_L over the copies + 0.1 p (0 when masked), into shared memory; then every
-// point as k_cg_update, c formed.  The boundary points come from a table
-// sorted by kind (faces, edges, corners): on GB300 an FP64 instruction costs
-// its warp the same whether one lane or all take part (two lanes a cycle and
-// SM), and the one-pass form, in which every warp holds a few boundary
-// points, took 1.33 ms at 32^3 (this one 0.40 / 0.66 ms for the two halves of
-// a pair; the FP64 pipe and HBM bound it).
+// FORM 1: a block takes an element at a time (FORM 2, below lx1 = 8: ne of
+// them, so many that it has a thousand points): first their boundary points, w = sum of w' over the copies (0 when masked), into shared memory;
+// then every point as k_cg_update, c formed.  The boundary points come from a
+// table sorted by kind (faces, edges, corners): on GB300 an FP64 instruction
+// costs its warp the same whether one lane or all take part (two lanes a
+// cycle and SM), and the one-pass form, in which every warp holds a few
+// boundary points, took 1.33 ms at 32^3 (this one 0.36 / 0.60 ms for the two
+// halves of a pair; the FP64 pipe and HBM bound it).
+// FORM 0, one pass, a thread a point: small meshes, where a block's two phases
+// and the few blocks are what takes the time (update_one_pass).
 // Where the solve's flag is off, w is already finished and this is
 // k_cg_update's loop.  VEC points a thread at a time (16 bytes) when every
 // vector is aligned and lx1 is even, else one.
-// (eight blocks per SM, 32 registers: 0.53 ms for the pair's average at 32^3
-// FP64 and 0.105 ms at 24^3 FP32, against 0.53 and 0.121 with five)
-template <typename T, int DEFER, int VEC>
+// (eight blocks per SM, 32 registers: 0.105 ms for the pair's average at 24^3
+// FP32 against 0.121 with five; FP64 the same)
+template <typename T, int DEFER, int VEC, int FORM>
 __global__ void __launch_bounds__(256, 8)
     k_cg_update_box(T *__restrict__ x, T *__restrict__ r, const T *__restrict__ p,
                     const T *__restrict__ w, const T *__restrict__ c, long n,
                     double *__restrict__ partial, unsigned *counter, CgScalars *sc,
-                    double *hist, int iter, const T *__restrict__ pprev, const BoxMesh box) {
+                    double *hist, int iter, const T *__restrict__ pprev, const BoxMesh box,
+                    int ne_) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ double red[32];
   struct alignas(VEC * sizeof(T)) Pack { T v[VEC]; };
   const bool whole = sc->box_ok != 0;
-  const int lx = box.lx, l3 = lx * lx * lx;
-  T *wb = reinterpret_cast<T *>(smem_raw);           // l3: w of the boundary points
-  unsigned char *ext = smem_raw + l3 * sizeof(T);    // l3: extreme bits
+  const int lx = box.lx, l3 = lx * lx * lx, ne = FORM == 2 ? ne_ : 1;
   const T alpha = T(sc->alpha);
   const T alphm = -alpha;
   const T alpha0 = DEFER == 2 ? T(sc->alpha_prev) : T(0);
@@ -865,48 +879,84 @@ __global__ void __launch_bounds__(256, 8)
     if (DEFER != 1) reinterpret_cast<Pack *>(x)[v] = xa;
     reinterpret_cast<Pack *>(r)[v] = ra;
   };
-  if (whole) {
-    for (int l = threadIdx.x; l < l3; l += blockDim.x)
-      ext[l] = (unsigned char)box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx);
-    const int Q = l3 / VEC, nelt = int(n / l3);
-    for (int e = blockIdx.x; e < nelt; e += gridDim.x) {
-      const unsigned nbr = box_neighbours(box, e);
-      const int base = e * l3;
+  // w at point l of element e, extreme bits ex, a boundary point
+  auto boundary_w = [&](int e, int l, unsigned ex, unsigned nbr) {
+    const unsigned cp = ex & nbr;
+    if (box_masked(box, e, l, ex, nbr)) return T(0);
+    const BoxCopies k = box_copies(box, e * l3 + l, cp);
+    T t = box_sum(w, k);
+    if (!box.full_mask) t = add_rn(t, box_missing(box, k, cp, p[e * l3 + l]));
+    return t;
+  };
+  auto load = [&](unsigned v, Pack &xa, Pack &pa, Pack &qa, Pack &ra) {
+    if (DEFER != 1) {
+      xa = reinterpret_cast<const Pack *>(x)[v];
+      pa = reinterpret_cast<const Pack *>(p)[v];
+    }
+    if (DEFER == 2) qa = reinterpret_cast<const Pack *>(pprev)[v];
+    ra = reinterpret_cast<const Pack *>(r)[v];
+  };
+  if (whole && FORM == 0) {
+    const unsigned nv = unsigned(n), vs = gridDim.x * blockDim.x;
+    for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += vs) {
+      Pack xa, ra, pa, wa, qa;
+      load(v, xa, pa, qa, ra);
+      wa = reinterpret_cast<const Pack *>(w)[v];
+      const int e = int(v / unsigned(l3)), l = int(v - unsigned(e * l3));
+      const unsigned nbr = box_neighbours(box, e), ex = __ldg(box.ext + l);
+      const int m[1] = {__popc(ex & nbr)};
+      if (ex) wa.v[0] = boundary_w(e, l, ex, nbr);
+      update(v, wa, xa, pa, qa, ra, m, nullptr);
+    }
+  } else if (whole) {
+    T *wb = reinterpret_cast<T *>(smem_raw);  // ne l3: w of the boundary points
+    // per point its extreme bits and its element of the ne, per element its faces
+    unsigned char *ext = smem_raw + ne * l3 * sizeof(T), *own = ext + ne * l3,
+                  *fnb = own + (FORM == 2 ? ne * l3 : 0);
+    for (int l = threadIdx.x; l < ne * l3; l += blockDim.x) {
+      const int el = l / l3;
+      ext[l] = __ldg(box.ext + (l - el * l3));
+      if (FORM == 2) own[l] = (unsigned char)el;
+    }
+    const int nelt = int(n / l3), nf = 6 * (lx - 2) * (lx - 2), nr = box.nbnd - nf;
+    for (int e0 = blockIdx.x * ne; e0 < nelt; e0 += gridDim.x * ne) {
+      const int nh = min(ne, nelt - e0), Q = nh * l3 / VEC;
+      const int base = e0 * l3;
+      if (FORM == 2)
+        for (int el = threadIdx.x; el < nh; el += blockDim.x)
+          fnb[el] = (unsigned char)box_neighbours(box, e0 + el);
+      unsigned nbr = box_neighbours(box, e0);
       // faces: one copy at most besides the point's own, no branches
-      const int nf = 6 * (lx - 2) * (lx - 2);
 #pragma unroll 3
-      for (int b = threadIdx.x; b < nf; b += blockDim.x) {
-        const unsigned u = __ldg(box.bnd + b);
+      for (int b = threadIdx.x; b < nh * nf; b += blockDim.x) {
+        const int el = FORM == 2 ? b / nf : 0, e = e0 + el;
+        if (FORM == 2) nbr = box_neighbours(box, e);
+        const unsigned u = __ldg(box.bnd + (b - el * nf));
         const int l = int(u & 0xFFFFu);
         const unsigned ex = u >> 16, cp = ex & nbr;
-        const BoxCopies c = box_copies(box, base + l, cp);
-        const int d = c.d0 + c.d1 + c.d2;
-        const T pv = p[base + l], a = w[c.q0], o = w[c.q0 + d];
-        const T t = fma_rn(T(0.1), pv, d ? add_rn(a, o) : a);
-        wb[l] = box_masked(box, e, l, ex, nbr) ? T(0) : t;
+        const BoxCopies k = box_copies(box, e * l3 + l, cp);
+        const int d = k.d0 + k.d1 + k.d2;
+        const T a = w[k.q0], o = w[k.q0 + d];
+        T t = d ? add_rn(a, o) : a;
+        if (!box.full_mask) t = add_rn(t, box_missing(box, k, cp, p[e * l3 + l]));
+        wb[el * l3 + l] = box_masked(box, e, l, ex, nbr) ? T(0) : t;
       }
-      for (int b = nf + threadIdx.x; b < box.nbnd; b += blockDim.x) {
-        const unsigned u = __ldg(box.bnd + b);
+      for (int b = threadIdx.x; b < nh * nr; b += blockDim.x) {
+        const int el = FORM == 2 ? b / nr : 0, e = e0 + el;
+        if (FORM == 2) nbr = box_neighbours(box, e);
+        const unsigned u = __ldg(box.bnd + nf + (b - el * nr));
         const int l = int(u & 0xFFFFu);
-        const unsigned ex = u >> 16, cp = ex & nbr;
-        const bool masked = box_masked(box, e, l, ex, nbr);
-        T t = T(0);
-        if (!masked) t = fma_rn(T(0.1), p[base + l], box_sum(w, box_copies(box, base + l, cp)));
-        wb[l] = t;
+        wb[el * l3 + l] = boundary_w(e, l, u >> 16, nbr);
       }
       __syncthreads();
       const int v0 = base / VEC;
       for (int v = threadIdx.x; v < Q; v += blockDim.x) {
         Pack xa, ra, pa, wa, qa;
         int m[VEC];
-        if (DEFER != 1) {
-          xa = reinterpret_cast<const Pack *>(x)[v0 + v];
-          pa = reinterpret_cast<const Pack *>(p)[v0 + v];
-        }
-        if (DEFER == 2) qa = reinterpret_cast<const Pack *>(pprev)[v0 + v];
-        ra = reinterpret_cast<const Pack *>(r)[v0 + v];
+        load(unsigned(v0 + v), xa, pa, qa, ra);
         wa = reinterpret_cast<const Pack *>(w)[v0 + v];
         const Pack ba = reinterpret_cast<const Pack *>(wb)[v];
+        if (FORM == 2) nbr = fnb[own[v * VEC]];
 #pragma unroll
         for (int q = 0; q < VEC; ++q) {
           const unsigned ex = ext[v * VEC + q];
@@ -921,12 +971,7 @@ __global__ void __launch_bounds__(256, 8)
     const unsigned nv = unsigned(n / VEC), vs = gridDim.x * blockDim.x;
     for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += vs) {
       Pack xa, ra, pa, wa, ca, qa;
-      if (DEFER != 1) {
-        xa = reinterpret_cast<const Pack *>(x)[v];
-        pa = reinterpret_cast<const Pack *>(p)[v];
-      }
-      if (DEFER == 2) qa = reinterpret_cast<const Pack *>(pprev)[v];
-      ra = reinterpret_cast<const Pack *>(r)[v];
+      load(v, xa, pa, qa, ra);
       wa = reinterpret_cast<const Pack *>(w)[v];
       ca = reinterpret_cast<const Pack *>(c)[v];
       update(v, wa, xa, pa, qa, ra, nullptr, &ca);
@@ -965,18 +1010,14 @@ __global__ void __launch_bounds__(256)
     k_box_begin(T *x, const T *f, T *r, const T *c, long n, double *__restrict__ partial,
                 unsigned *counter, CgScalars *sc, double *hist, const BoxMesh box) {
   __shared__ double red[32];
-  __shared__ unsigned char ext[4096];
   const int lx = box.lx, l3 = lx * lx * lx;
-  for (int l = threadIdx.x; l < l3; l += blockDim.x)
-    ext[l] = (unsigned char)box_ext(l % lx, (l / lx) % lx, l / (lx * lx), lx);
-  __syncthreads();
   const unsigned q0 = blockIdx.x * blockDim.x + threadIdx.x, qs = gridDim.x * blockDim.x;
   int e = int(q0 / l3), l = int(q0 % l3);
   const int se = int(qs / l3), sl = int(qs % l3);
   T part = T(0);
   bool ok = true;
   for (long q = q0; q < n; q += qs) {
-    const unsigned nbr = box_neighbours(box, e), ex = ext[l], cp = ex & nbr;
+    const unsigned nbr = box_neighbours(box, e), ex = __ldg(box.ext + l), cp = ex & nbr;
     const T fv = f[q], cv = c[q];
     const bool masked = ex && box_masked(box, e, l, ex, nbr);
     const T rv = masked ? T(0) : fv;
@@ -1028,9 +1069,11 @@ __global__ void __launch_bounds__(256)
     const int b = off[g], e = off[g + 1];
     T t = w[idx[b] & 0x7fffffffu];
     for (int q = b + 1; q < e; ++q) t = add_rn(t, w[idx[q] & 0x7fffffffu]);
+    // (box_missing's term)
+    const T ms = (idx[b] & 0x80000000u) ? T(0.1) / T(e - b) : T(0);
     for (int q = b; q < e; ++q) {
       const unsigned m = idx[q], id = m & 0x7fffffffu;
-      w[id] = (m & 0x80000000u) ? T(0) : fma_rn(T(0.1), p[id], t);
+      w[id] = (m & 0x80000000u) ? T(0) : fma_rn(ms, p[id], t);
     }
   }
 }
@@ -1544,9 +1587,8 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
     const bool interior = col_interior && (k > 0) && (k < LX - 1);
     if (MODE == 1) {
       if (whole) {
-        const T wv = fma_rn(box_tenth<T>(box_ext<LX>(i, j, k) & nbr), ureg[k], wl);
-        part = fma_rn(wv, ureg[k], part);
-        if (interior) wl = wv;
+        wl = fma_rn(box_tenth<T>(box_ext<LX>(i, j, k) & nbr), ureg[k], wl);
+        part = fma_rn(wl, ureg[k], part);
       } else if (interior) {
         wl = fma_rn(T(0.1), ureg[k], wl);
         part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);

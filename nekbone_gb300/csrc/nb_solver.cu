@@ -24,16 +24,12 @@ namespace nb {
 
 Operator::~Operator() {
   if (dD) cudaFree(dD);
-  if (fD) cudaFree(fD);
   gs_release(&gs);
   if (d_mask_list) cudaFree(d_mask_list);
-  if (d_face) cudaFree(d_face);
   if (bnd_off) cudaFree(bnd_off);
   if (bnd_idx) cudaFree(bnd_idx);
   if (gfx) cudaFree(gfx);
-  if (gexp) cudaFree(gexp);
-  if (d_mask0) cudaFree(d_mask0);
-  if (d_bnd_pts) cudaFree(d_bnd_pts);
+  if (sep) cudaFree(sep);
 }
 
 BoxMesh Operator::box_mesh() const {
@@ -48,6 +44,7 @@ BoxMesh Operator::box_mesh() const {
   b.mask0 = d_mask0;
   b.bnd = d_bnd_pts;
   b.nbnd = n_bnd_pts;
+  b.ext = reinterpret_cast<const unsigned char *>(d_bnd_pts + n_bnd_pts);
   return b;
 }
 
@@ -384,7 +381,6 @@ int operator_set_mask(Operator *op, const std::vector<int> &list_in) {
   if (op->box_groups && op->mask_mode == 0 && (list.empty() || list.back() < l3)) {
     std::vector<unsigned char> m0(l3, 0);
     for (int v : list) m0[v] = 1;
-    if (!op->d_mask0) NB_CUDA(cudaMalloc(&op->d_mask0, l3));
     NB_CUDA(cudaMemcpy(op->d_mask0, m0.data(), l3, cudaMemcpyHostToDevice));
     op->mask0_ok = true;
   }
@@ -432,11 +428,6 @@ int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
   op->lglel.assign(lglel, lglel + nelt);
   op->D.assign(dxm1, dxm1 + lx * lx);
   op->mask_mode = mask_mode;
-  NB_CUDA(cudaMalloc(&op->dD, lx * lx * sizeof(double)));
-  NB_CUDA(cudaMalloc(&op->fD, lx * lx * sizeof(float)));
-  std::vector<float> fDh(op->D.begin(), op->D.end());
-  NB_CUDA(cudaMemcpy(op->dD, op->D.data(), lx * lx * sizeof(double), cudaMemcpyHostToDevice));
-  NB_CUDA(cudaMemcpy(op->fD, fDh.data(), lx * lx * sizeof(float), cudaMemcpyHostToDevice));
   // even-odd tables when D(n-1-i,n-1-m) = -D(i,m) holds to rounding
   op->eo_ok = even_odd_tables(op->D, lx, op->EO);
   op->fx_ok = anti_centrosymmetric(op->D, lx) &&
@@ -454,14 +445,28 @@ int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
     for (int f = 1; f < 64; ++f)
       if (__builtin_popcount(f) == kind) pts.insert(pts.end(), of[f].begin(), of[f].end());
   op->n_bnd_pts = int(pts.size());
-  NB_CUDA(cudaMalloc(&op->d_bnd_pts, pts.size() * sizeof(unsigned)));
-  NB_CUDA(cudaMemcpy(op->d_bnd_pts, pts.data(), pts.size() * sizeof(unsigned),
-                     cudaMemcpyHostToDevice));
+  // one allocation: D in both precisions, these points, every point's bits,
+  // room for element 0's mask, the elements' domain faces
+  const size_t l2 = size_t(lx) * lx, l3 = l2 * lx;
   op->face.resize(nelt);
   for (int e = 0; e < nelt; ++e)
     op->face[e] = (unsigned char)face_bits(op->lglel[e], nelx, nely, nelz);
-  NB_CUDA(cudaMalloc(&op->d_face, nelt));
-  NB_CUDA(cudaMemcpy(op->d_face, op->face.data(), nelt, cudaMemcpyHostToDevice));
+  std::vector<unsigned char> h(12 * l2 + 4 * pts.size() + 2 * l3 + nelt, 0);
+  const std::vector<float> fDh(op->D.begin(), op->D.end());
+  unsigned char *hp = h.data() + 12 * l2, *ext = hp + 4 * pts.size();
+  std::memcpy(h.data(), op->D.data(), 8 * l2);
+  std::memcpy(h.data() + 8 * l2, fDh.data(), 4 * l2);
+  std::memcpy(hp, pts.data(), 4 * pts.size());
+  for (unsigned u : pts) ext[u & 0xFFFFu] = (unsigned char)(u >> 16);
+  std::copy(op->face.begin(), op->face.end(), ext + 2 * l3);
+  unsigned char *d = nullptr;
+  NB_CUDA(cudaMalloc(&d, h.size()));
+  op->dD = reinterpret_cast<double *>(d);  // (the allocation's owner)
+  op->fD = reinterpret_cast<float *>(d + 8 * l2);
+  op->d_bnd_pts = reinterpret_cast<unsigned *>(d + 12 * l2);
+  op->d_mask0 = d + (ext - h.data()) + l3;
+  op->d_face = op->d_mask0 + l3;
+  NB_CUDA(cudaMemcpy(d, h.data(), h.size(), cudaMemcpyHostToDevice));
   return NB_OK;
 }
 
@@ -625,16 +630,39 @@ int c_closed_form(const Operator &op, const float *c32, unsigned char *cface, in
 }
 
 namespace {
-// the resident blocks of k_cg_update_box: its grid is one wave
-template <typename T, int D, int VEC>
-int update_box_blocks(int lx, int nt, size_t sm) {
-  static int cached[kMaxLx + 1] = {0};
-  if (!cached[lx]) {
+// Whether a mesh is small enough for k_cg_update_box's one-pass form: 20 CG
+// iterations on 3^3 elements, lx1 = 16, 832 us against 998, on 7^3, lx1 = 10
+// (343,000 points), 883 against 859; the mixed solve's FP32 iteration gains to
+// about twice that size (12^3 points by 6^3 elements: 3.47 ms against 3.78).
+template <typename T>
+bool update_one_pass(const Operator &op) {
+  const long n = sizeof(T) == 8 ? 200000 : 600000;
+  return op.n <= n || (op.nelt < 152 && op.n <= 600000);
+}
+
+// k_cg_update_box in one form: its grid is one wave of resident blocks
+template <typename T, int D, int VEC, int FORM>
+void update_box_launch(const Operator &op, const CgWork &wk, T *x, T *r, const T *p,
+                       const T *w, const T *c, double *hist, int iter, const T *pprev,
+                       cudaStream_t s) {
+  const int l3 = op.lx * op.lx * op.lx;
+  // elements a block takes at a time (as many small ones as make 1000 points);
+  // threads: as many as take the packs in equal turns of at most 256
+  const int ne = FORM == 2 ? std::max(1, 1000 / l3) : 1;
+  const int Q = ne * l3 / VEC, turns = (Q + 255) / 256;
+  const int nt = FORM == 0 ? 256 : std::max(32, (Q / turns + 31) / 32 * 32);
+  const size_t sm = FORM == 0 ? 0 : size_t(ne) * l3 * (sizeof(T) + (FORM == 2 ? 2 : 1)) + (FORM == 2 ? ne : 0);
+  static int resident[kMaxLx + 1] = {0};
+  if (!resident[op.lx]) {
     int b = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_update_box<T, D, VEC>, nt, sm);
-    cached[lx] = sm_count() * std::max(1, b);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_cg_update_box<T, D, VEC, FORM>, nt, sm);
+    resident[op.lx] = sm_count() * std::max(1, b);
   }
-  return cached[lx];
+  const long units = FORM == 0 ? (op.n + nt - 1) / nt : (op.nelt + ne - 1) / ne;
+  const int grid = int(std::min<long>(std::min(wk.grid_up, resident[op.lx]), units));
+  k_cg_update_box<T, D, VEC, FORM><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
+                                                        wk.counters + 1, wk.sc, hist, iter,
+                                                        pprev, wk.box, ne);
 }
 
 // The third kernel of an iteration, pairing mode D: the assembled update on
@@ -649,22 +677,14 @@ void update_launch(const Operator &op, const CgWork &wk, T *x, T *r, const T *p,
     const uintptr_t al = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(r) |
                          reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(w) |
                          reinterpret_cast<uintptr_t>(c) | reinterpret_cast<uintptr_t>(pprev);
-    // threads: as many as take the element's packs in equal turns of at most 256
-    const bool vec = (al & 15u) == 0 && op.lx % 2 == 0;
-    const int l3 = op.lx * op.lx * op.lx, Q = vec ? l3 / VEC : l3;
-    const int nt = std::max(32, (Q / ((Q + 255) / 256) + 31) / 32 * 32);
-    const size_t sm = size_t(l3) * (sizeof(T) + 1);
-    const int grid = std::min(std::min(wk.grid_up, std::max(op.nelt, 1)),
-                              vec ? update_box_blocks<T, D, VEC>(op.lx, nt, sm)
-                                  : update_box_blocks<T, D, 1>(op.lx, nt, sm));
-    if (vec)
-      k_cg_update_box<T, D, VEC><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
-                                                      wk.counters + 1, wk.sc, hist, iter,
-                                                      pprev, wk.box);
+    if (update_one_pass<T>(op))
+      update_box_launch<T, D, 1, 0>(op, wk, x, r, p, w, c, hist, iter, pprev, s);
+    else if ((al & 15u) == 0 && op.lx % 2 == 0)
+      op.lx < 8 ? update_box_launch<T, D, VEC, 2>(op, wk, x, r, p, w, c, hist, iter, pprev, s)
+                : update_box_launch<T, D, VEC, 1>(op, wk, x, r, p, w, c, hist, iter, pprev, s);
     else
-      k_cg_update_box<T, D, 1><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
-                                                    wk.counters + 1, wk.sc, hist, iter, pprev,
-                                                    wk.box);
+      op.lx < 8 ? update_box_launch<T, D, 1, 2>(op, wk, x, r, p, w, c, hist, iter, pprev, s)
+                : update_box_launch<T, D, 1, 1>(op, wk, x, r, p, w, c, hist, iter, pprev, s);
     return;
   }
   if constexpr (std::is_same<T, float>::value) {
@@ -787,15 +807,16 @@ static bool box_form(const Operator &op) {
 }
 
 // cg.f:36-42: x = 0, r = mask(f), rnorm = sqrt(glsc3(r,c,r)).  plain: the
-// solve runs the fused iteration without preconditioner.
+// solve runs the fused iteration without preconditioner; unfused: it runs the
+// unfused one by request.
 template <typename T>
 static int cg_begin_t(Operator &op, CgWork &wk, T *x, const T *f, const T *c,
-                      T *r, bool plain, int niter, cudaStream_t s) {
+                      T *r, bool plain, int niter, cudaStream_t s, bool unfused = false) {
   const long n = op.n;
   NB_TRY(wk.ensure(op, niter));
   wk.r32_ready = false;
   wk.box = BoxMesh{};
-  if (std::is_same<T, double>::value) metric_fx_invalidate(op);
+  if (std::is_same<T, double>::value) metric_fx_invalidate(op, op.fused_ok && !unfused);
   // the reference's list is built by its first mask (of r, below)
   const bool built = op.mask_built || op.mask_mode == 1;
   if (!built || !plain || !box_form<T>(op)) {
@@ -1042,7 +1063,7 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
               const double *g, const double *c, double *r, double *w,
               double *p, double *z, int niter, Precond *M, bool force_unfused,
               cudaStream_t s) {
-  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, !M && !force_unfused, niter, s));
+  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, !M && !force_unfused, niter, s, force_unfused));
   // the second direction buffer of the paired x update (fused, no
   // preconditioner, at least one pair)
   double *p_alt = nullptr;

@@ -33,6 +33,9 @@ struct Operator {
   // gfx_src
   mutable int2 *gfx = nullptr;
   mutable int *gexp = nullptr;
+  mutable fx::SepTables *sep = nullptr;  // its separable form (even lx only),
+  mutable bool sep_on = false;           //   looked for in this solve
+  mutable bool metric_solve = false;
   mutable const double *gfx_src = nullptr;
   mutable long gfx_cap = 0;
   int order = 2;                   // 0 reference left-to-right sums, 1 even-odd
@@ -62,7 +65,7 @@ struct Operator {
   bool box_groups = false;           // the boundary groups are a brick box's copies
   unsigned char *d_mask0 = nullptr;  // a box's mask list as flags of element 0's points
   bool mask0_ok = false;             //   (no other element masked)
-  unsigned *d_bnd_pts = nullptr;     // BoxMesh::bnd
+  unsigned *d_bnd_pts = nullptr;     // BoxMesh::bnd (and, behind it, ::ext and mask0)
   int n_bnd_pts = 0;
   // the box for the assembled update (nb_kernels.cuh); nx = 0 where the mesh
   // or its mask is not of that form
@@ -129,11 +132,14 @@ bool even_odd_tables(const std::vector<double> &D, int lx, std::vector<double> &
 bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
                std::vector<int> &lo, std::vector<int> &d, int *fc);
 // The metric g in the fixed-point operator's form, converted when g is not
-// the array last converted (one pass over g); metric_fx_invalidate forgets
+// the array last converted: the separable form where g has it (op.sep),
+// else op.gfx / op.gexp (one pass over g each, decided on the device);
+// metric_fx_invalidate forgets
 // the conversion (every solve and every standalone apply starts with it, so
-// a caller may change g's contents between calls).
-int metric_fx_prepare(const Operator &op, const double *g, cudaStream_t s);
-void metric_fx_invalidate(const Operator &op);
+// a caller may change g's contents between calls); solve: several fused
+// applies (modes 1 and 2) follow, and the separable form is looked for.
+int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s);
+void metric_fx_invalidate(const Operator &op, bool solve);
 // The mesh-independent part of an operator: sizes, element numbers, D and
 // its even-odd tables, the domain faces of every element.
 int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
