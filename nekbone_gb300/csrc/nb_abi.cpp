@@ -531,7 +531,7 @@ void ax_(double *w, const double *u, const double *gxyz, double *ur,
   double *dw, *du, *dg;
   if (dbuf(0, nn, &dw) || dbuf(1, nn, &du) || dbuf(2, 6 * nn, &dg)) return;
   if (h2d(du, u, nn * 8) || h2d(dg, gxyz, 6 * nn * 8)) return;
-  metric_fx_invalidate(*op, false);
+  metric_fx_single(*op);
   if (apply_ax<double>(*op, dw, du, dg, S.s)) return;
   if (d2h(w, dw, nn * 8)) return;
   if (sync()) return;
@@ -956,7 +956,7 @@ int nb_rhs_uniform(nb_mesh *mesh, double *f, const double *c, uint64_t seed) {
 int nb_ax(nb_mesh *mesh, double *w, const double *u, const double *g) {
   clear_status();
   if (!mesh) return fail(NB_ERR_HANDLE, "null mesh");
-  metric_fx_invalidate(mesh->op, false);
+  metric_fx_single(mesh->op);
   NB_TRY(apply_ax<double>(mesh->op, w, u, g, st().s));
   return NB_OK;
 }
@@ -964,7 +964,7 @@ int nb_ax(nb_mesh *mesh, double *w, const double *u, const double *g) {
 int nb_dssum(nb_mesh *mesh, void *u, int dom) {
   clear_status();
   if (!mesh) return fail(NB_ERR_HANDLE, "null mesh");
-  return gs_exec(mesh->op.gs, u, dom, 1, 0, st().s);
+  return dssum_dev(mesh->op, u, dom, st().s);
 }
 
 int nb_cg(nb_mesh *mesh, double *x, const double *f, const double *g,

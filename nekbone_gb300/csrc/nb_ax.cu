@@ -17,6 +17,7 @@ int launch_ax_f32_m2(int lx, AxArgs<float> a, cudaStream_t s);
 int launch_ax_fx_m0(const Operator &op, AxArgs<double> a, cudaStream_t s);
 int launch_ax_fx_m1(const Operator &op, AxArgs<double> a, cudaStream_t s);
 int launch_ax_fx_m2(const Operator &op, AxArgs<double> a, cudaStream_t s);
+int launch_ax_fx_m3(const Operator &op, AxArgs<double> a, cudaStream_t s);
 
 template <>
 int launch_ax<double>(const Operator &op, int mode, AxArgs<double> a, cudaStream_t s) {
@@ -25,6 +26,9 @@ int launch_ax<double>(const Operator &op, int mode, AxArgs<double> a, cudaStream
   a.err = device_error_word();
   a.wait_test = wait_test_mode();
   if (op.order == 2 && op.fx_ok) {  // fixed point on the integer pipes
+    // a single apply (metric_fx_single) converts the metric as it goes
+    if (mode == 0 && op.metric_single && (reinterpret_cast<uintptr_t>(a.g) & 15u) == 0)
+      return launch_ax_fx_m3(op, a, s);
     NB_TRY(metric_fx_prepare(op, a.g, op.dD, s));
     a.gfx = op.gfx;
     a.gexp = op.gexp;

@@ -291,6 +291,11 @@ bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
 void metric_fx_invalidate(const Operator &op, bool solve) {
   op.gfx_src = nullptr;
   op.metric_solve = solve;
+  op.metric_single = false;
+}
+void metric_fx_single(const Operator &op) {
+  metric_fx_invalidate(op, false);
+  op.metric_single = true;
 }
 
 int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s) {

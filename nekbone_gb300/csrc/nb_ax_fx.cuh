@@ -316,7 +316,7 @@ struct FxShared {
   i64 A[N];
   i64 C[N];
   i64 D[N];
-  int emax[8];
+  int emax[8], gmax[8];
   unsigned orl[8], orh[8];
   double red[32];
 };
@@ -445,15 +445,15 @@ __device__ __forceinline__ double ax_fx_finish(const AxArgs<double> &a, int e, i
   const bool col_interior = (i > 0) && (i < LX - 1) && (j > 0) && (j < LX - 1);
   double part = 0.0;
   double pk[NK], ck[NK], fk[NK];
-  if (WHOLE || (MODE != 0 && col_interior)) {
+  if (WHOLE || ((MODE == 1 || MODE == 2 || a.tenth) && col_interior)) {
 #pragma unroll
     for (int q = 0; q < NK; ++q) {  // all loads before the first store
       const int k = k0 + q;
       if (k >= LX) break;
       const size_t id = base + size_t(k) * L2 + t;
       const bool interior = k > 0 && k < LX - 1;
-      if (WHOLE || interior) pk[q] = a.p[id];
-      if (!WHOLE && interior) ck[q] = __ldg(a.c + id);
+      if (WHOLE || interior) pk[q] = MODE == 1 || MODE == 2 ? a.p[id] : a.u[id];
+      if (!WHOLE && interior && (MODE == 1 || MODE == 2)) ck[q] = __ldg(a.c + id);
       if (MODE == 2 && interior) fk[q] = __ldg(a.f + id);
     }
   }
@@ -484,6 +484,7 @@ __device__ __forceinline__ double ax_fx_finish(const AxArgs<double> &a, int e, i
         a.w[id] = wl;
       }
     } else {
+      if (a.tenth && interior) wl = fma_rn(0.1, pk[q], wl);
       a.w[id] = wl;
     }
   }
@@ -594,7 +595,12 @@ __device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX
   if (t == 0) a.partial[e] = s;
 }
 
-// MODE 0 / 1 / 2 as k_ax_eo (AxArgs); a.gfx / a.gexp hold the metric in
+// MODE 0 / 1 / 2 as k_ax_eo (AxArgs), 3 as 0 from the metric a.g itself: the
+// element's largest exponent first (its block read once, from L2 the second
+// time), each value converted where it is used.  For a single apply: the
+// conversion pass and its traffic (96 B a point written and read back) cost
+// more than these 100 instructions a point (16^3, lx1 = 12: 247 us against 160
+// for the conversion and 189 for mode 0).  a.gfx / a.gexp hold the metric in
 // fixed point (metric_fx_prepare).
 template <int LX, int MODE>
 __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef<LX> &cf) {
@@ -609,7 +615,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   if (a.act && !a.act[size_t(a.el_prob[e]) * a.act_stride]) return;  // the whole CTA
   const bool whole = MODE == 1 && box_flag(a.box_ok);  // pap formed here (BoxMesh)
   const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
-  if constexpr (MODE != 0 && !FxCoef<LX>::FULL) {
+  if constexpr ((MODE == 1 || MODE == 2) && !FxCoef<LX>::FULL) {
     const int2 sep = a.sep ? *reinterpret_cast<const int2 *>(a.sep) : make_int2(0, 0);
     if (sep.x) {
       ax_sep_body<LX, MODE>(a, sm, whole, nbr, sep.y);
@@ -653,6 +659,18 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     const int w = t >> 5;
     const int r = __reduce_max_sync(warp_mask(L2, w), unsigned(em));
     if ((t & 31) == 0) sm.emax[w] = r;
+    if constexpr (MODE == 3) {
+      // (values in any order: the block's 3 lx1 pairs a thread, coalesced)
+      const int4 *gp = reinterpret_cast<const int4 *>(a.g + 6 * base);
+      int ge = 0;
+#pragma unroll 6
+      for (int q = 0; q < 3 * LX; ++q) {
+        const int4 v = __ldg(gp + q * L2 + t);
+        ge = max(ge, max(v.y & 0x7FF00000, v.w & 0x7FF00000));
+      }
+      const int rg = __reduce_max_sync(warp_mask(L2, w), unsigned(ge));
+      if ((t & 31) == 0) sm.gmax[w] = rg;
+    }
     __syncthreads();
     em = 0;
     for (int q = 0; q < (L2 + 31) / 32; ++q) em = max(em, sm.emax[q]);
@@ -696,7 +714,13 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   const int sU = sP - fc + 64 - s1;  // ur = UR 2^sU after the shift
 
   // metric (cg.f:156-163) at the thread's own points, in place
-  const int eg = a.gexp[e];
+  int eg = 0;
+  if constexpr (MODE == 3) {
+    for (int q = 0; q < (L2 + 31) / 32; ++q) eg = max(eg, sm.gmax[q]);
+    eg >>= 20;
+  } else {
+    eg = a.gexp[e];
+  }
   const int sW = 64 - MK + (eg - 1082) + sU;  // wr = WR 2^sW before renormalising
   orv = 0;
 #pragma unroll 4
@@ -704,10 +728,22 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     const int q = fx_at<LX>(i, j, k);
     const Sp ur = split(shift_up(sm.A[q], s1)), us = split(shift_up(sm.C[q], s1)),
              ut = split(shift_up(sm.D[q], s1));
-    const int4 *gp = reinterpret_cast<const int4 *>(a.gfx + 6 * (base + size_t(k) * L2 + t));
-    const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
-    const Sp G1 = {g01.x, g01.y}, G2 = {g01.z, g01.w}, G3 = {g23.x, g23.y},
-             G4 = {g23.z, g23.w}, G5 = {g45.x, g45.y}, G6 = {g45.z, g45.w};
+    Sp G1, G2, G3, G4, G5, G6;
+    if constexpr (MODE == 3) {
+      const double2 *gp = reinterpret_cast<const double2 *>(a.g + 6 * (base + size_t(k) * L2 + t));
+      const double2 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
+      G1 = split(to_fixed60(g01.x, eg));
+      G2 = split(to_fixed60(g01.y, eg));
+      G3 = split(to_fixed60(g23.x, eg));
+      G4 = split(to_fixed60(g23.y, eg));
+      G5 = split(to_fixed60(g45.x, eg));
+      G6 = split(to_fixed60(g45.y, eg));
+    } else {
+      const int4 *gp = reinterpret_cast<const int4 *>(a.gfx + 6 * (base + size_t(k) * L2 + t));
+      const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
+      G1 = Sp{g01.x, g01.y}, G2 = Sp{g01.z, g01.w}, G3 = Sp{g23.x, g23.y};
+      G4 = Sp{g23.z, g23.w}, G5 = Sp{g45.x, g45.y}, G6 = Sp{g45.z, g45.w};
+    }
     Acc<MK> wr, ws, wt;
     wr.mac(G1, ur); wr.mac(G2, us); wr.mac(G3, ut);
     ws.mac(G2, ur); ws.mac(G4, us); ws.mac(G5, ut);
@@ -753,7 +789,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     part = ax_fx_finish<LX, MODE, LX, MODE == 1>(a, e, t, 0, bad, nbr, wloc);
   else
     part = ax_fx_finish<LX, MODE, LX, false>(a, e, t, 0, bad, nbr, wloc);
-  if (MODE != 0) {
+  if (MODE == 1 || MODE == 2) {
     const double s = block_sum<double>(part, sm.red);
     if (t == 0) a.partial[e] = s;
   }

@@ -253,6 +253,7 @@ struct AxArgs {
   int act_stride;      //   problem is no longer active); null for one mesh
   int c_unit_interior;  // MODE 1: c is 1 at every element-interior point (a
                         //   verified multiplicity): not read there
+  int tenth;           // MODE 0 (and 3): interior points get w_L + 0.1 u (ax, cg.f:119)
   BoxMesh box;         // MODE 1, with box_ok (the solve's flag; null: general form):
   const int *box_ok;   //   partial is the element's whole part of pap
 };
@@ -474,6 +475,7 @@ __global__ void __launch_bounds__(LX * LX)
         a.w[id] = wl;
       }
     } else {
+      if (a.tenth && interior) wl = fma_rn(T(0.1), ureg[k], wl);
       a.w[id] = wl;
     }
   }
@@ -854,7 +856,7 @@ __global__ void __launch_bounds__(256, 8)
                     double *__restrict__ partial, unsigned *counter, CgScalars *sc,
                     double *hist, int iter, const T *__restrict__ pprev, const BoxMesh box,
                     int ne_) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
+  extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ double red[32];
   struct alignas(VEC * sizeof(T)) Pack { T v[VEC]; };
   const bool whole = sc->box_ok != 0;
@@ -1054,6 +1056,61 @@ __global__ void __launch_bounds__(256)
         hist[0] = sc->rnorm;
         hist[1] = hist[2] = hist[3] = hist[4] = 0.0;
       }
+    }
+  }
+}
+
+// The boundary points of a box in place, in closed form: t = sum of w over the
+// copies in jl's order, then every copy gets t (AX false: dssum,
+// prox_dssum.f:2-12) or t + 0.1 u, 0 when masked (AX: the rest of ax,
+// cg.f:117-120, after an operator with `tenth`).  A thread takes a point's
+// lowest copy; the boundary points come kind by kind (BoxMesh::bnd), so a
+// warp's threads mostly do the same, and whole warps skip the faces whose
+// points have a lower copy.  Bound by the latency of its gathers, as the
+// group lists' pass: ax at 16^3, lx1 = 12 in FP64 31 us, where the
+// gather-scatter, add2s2 and mask passes took 25 + 23 + 4.
+template <typename T, bool AX>
+__global__ void __launch_bounds__(256)
+    k_box_assemble(T *__restrict__ w, const T *__restrict__ u, const BoxMesh box,
+                   unsigned total) {
+  const unsigned l3 = unsigned(box.lx * box.lx * box.lx);
+#pragma unroll 2
+  for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < total;
+       v += gridDim.x * blockDim.x) {
+    const unsigned e = v / unsigned(box.nbnd), b = v - e * unsigned(box.nbnd);
+    const unsigned en = __ldg(box.bnd + b), ex = en >> 16, nbr = box_neighbours(box, int(e));
+    const unsigned cp = ex & nbr;
+    if ((cp & 21u) || (!AX && !cp)) continue;  // a lower copy's, or alone
+    const int q = int(e * l3 + (en & 0xFFFFu));
+    const BoxCopies k = box_copies(box, q, cp);
+    const T t = box_sum(w, k);
+    const bool all = AX && box.full_mask && (ex & ~nbr) != 0u;
+    const bool own = AX && !box.full_mask && e == 0u && box.mask0[en & 0xFFFFu] != 0;
+    const unsigned have = (k.d0 ? 2u : 0u) | (k.d1 ? 4u : 0u) | (k.d2 ? 16u : 0u);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      const unsigned need = (m & 1 ? 2u : 0u) | (m & 2 ? 4u : 0u) | (m & 4 ? 16u : 0u);
+      if (need & ~have) continue;
+      const int id = q + (m & 1 ? k.d0 : 0) + (m & 2 ? k.d1 : 0) + (m & 4 ? k.d2 : 0);
+      T r = t;
+      if (AX) r = all || (own && m == 0) ? T(0) : fma_rn(T(0.1), u[id], t);
+      w[id] = r;
+    }
+  }
+}
+
+// The same rest of ax for any mesh, from the boundary groups.
+template <typename T>
+__global__ void __launch_bounds__(256)
+    k_ax_rest(T *__restrict__ w, const T *__restrict__ u, const int *__restrict__ off,
+              const unsigned *__restrict__ idx, int ng) {
+  for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
+    const int b = off[g], e = off[g + 1];
+    T t = w[idx[b] & 0x7fffffffu];
+    for (int q = b + 1; q < e; ++q) t = add_rn(t, w[idx[q] & 0x7fffffffu]);
+    for (int q = b; q < e; ++q) {
+      const unsigned m = idx[q], id = m & 0x7fffffffu;
+      w[id] = (m & 0x80000000u) ? T(0) : fma_rn(T(0.1), u[id], t);
     }
   }
 }
@@ -1280,10 +1337,10 @@ __global__ void __launch_bounds__(LX * LX)
     const float tt = dot_contig<float, LX>(wtreg, &sm.Dc[k * LX]);
     float wl = add_rn(add_rn(tr, ts), tt);
     const size_t id = base + size_t(k) * L2 + tid;
-    if (MODE == 1) {
+    if (MODE == 1 || a.tenth) {
       if (col_interior && k > 0 && k < LX - 1) {
         wl = fma_rn(0.1f, ureg[k], wl);
-        part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);
+        if (MODE == 1) part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);
       }
     }
     a.w[id] = wl;
@@ -1603,6 +1660,7 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
         a.w[id] = wl;
       }
     } else {
+      if (a.tenth && interior) wl = fma_rn(T(0.1), ureg[k], wl);
       a.w[id] = wl;
     }
   }

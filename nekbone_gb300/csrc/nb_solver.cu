@@ -33,8 +33,13 @@ Operator::~Operator() {
 }
 
 BoxMesh Operator::box_mesh() const {
+  if (!fused_ok || !mask_built || (mask_mode != 1 && !mask0_ok)) return BoxMesh{};
+  return box_shape();
+}
+
+BoxMesh Operator::box_shape() const {
   BoxMesh b{};
-  if (!box_groups || !fused_ok || !mask_built || (mask_mode != 1 && !mask0_ok)) return b;
+  if (!box_groups) return b;
   b.nx = nelx;
   b.ny = nely;
   b.nz = nelz;
@@ -780,6 +785,31 @@ static int maskit_dev(Operator &op, T *w, cudaStream_t s) {
   return vec_mask<T>(w, op.d_mask_list, op.n_mask, s);
 }
 
+// the boundary points of a box in place (k_box_assemble)
+template <typename T, bool AX>
+static int box_assemble(const Operator &op, const BoxMesh &b, T *w, const T *u, cudaStream_t s) {
+  static int resident = 0;
+  if (!resident) {
+    int k = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_box_assemble<T, AX>, 256, 0);
+    resident = sm_count() * std::max(1, k);
+  }
+  const long total = long(op.nelt) * b.nbnd;  // below n
+  const int grid = int(std::max(1L, std::min<long>(resident, (total + 255) / 256)));
+  k_box_assemble<T, AX><<<grid, 256, 0, s>>>(w, u, b, unsigned(total));
+  NB_CUDA(cudaGetLastError());
+  return NB_OK;
+}
+
+int dssum_dev(const Operator &op, void *u, int dom, cudaStream_t s) {
+  const BoxMesh b = op.box_shape();
+  if (b.nx > 0 && dom == 1)
+    return box_assemble<double, false>(op, b, static_cast<double *>(u), nullptr, s);
+  if (b.nx > 0 && dom == 2)
+    return box_assemble<float, false>(op, b, static_cast<float *>(u), nullptr, s);
+  return gs_exec(op.gs, u, dom, 1, 0, s);
+}
+
 template <typename T>
 int apply_ax(const Operator &op_c, T *w, const T *u, const T *g, cudaStream_t s) {
   Operator &op = const_cast<Operator &>(op_c);
@@ -788,7 +818,17 @@ int apply_ax(const Operator &op_c, T *w, const T *u, const T *g, cudaStream_t s)
   a.u = u;
   a.g = g;
   a.D = std::is_same<T, double>::value ? (const T *)op.dD : (const T *)op.fD;
+  // two passes where the boundary groups and the mask are at hand (and w is
+  // not u itself, which the second pass reads), else four
+  a.tenth = op.fused_ok && (op.mask_built || op.mask_mode == 1) && w != u ? 1 : 0;
   NB_TRY(launch_ax<T>(op, 0, a, s));
+  if (a.tenth) {
+    const BoxMesh b = op.box_mesh();
+    if (b.nx > 0) return box_assemble<T, true>(op, b, w, u, s);
+    k_ax_rest<T><<<grid_for(op.nbg), 256, 0, s>>>(w, u, op.bnd_off, op.bnd_idx, op.nbg);
+    NB_CUDA(cudaGetLastError());
+    return NB_OK;
+  }
   NB_TRY(gs_exec(op.gs, w, std::is_same<T, double>::value ? 1 : 2, 1, 0, s));
   NB_TRY(vec_add2s2<T>(w, u, 0.1, op.n, s));
   return maskit_dev<T>(op, w, s);

@@ -36,6 +36,7 @@ struct Operator {
   mutable fx::SepTables *sep = nullptr;  // its separable form (even lx only),
   mutable bool sep_on = false;           //   looked for in this solve
   mutable bool metric_solve = false;
+  mutable bool metric_single = false;    // one plain apply: no conversion pass
   mutable const double *gfx_src = nullptr;
   mutable long gfx_cap = 0;
   int order = 2;                   // 0 reference left-to-right sums, 1 even-odd
@@ -70,6 +71,7 @@ struct Operator {
   // the box for the assembled update (nb_kernels.cuh); nx = 0 where the mesh
   // or its mask is not of that form
   BoxMesh box_mesh() const;
+  BoxMesh box_shape() const;        // the same without the mask's conditions
 
   ~Operator();
 };
@@ -140,6 +142,8 @@ bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
 // applies (modes 1 and 2) follow, and the separable form is looked for.
 int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s);
 void metric_fx_invalidate(const Operator &op, bool solve);
+// The same before a single plain apply (apply_ax<double>, mode 0).
+void metric_fx_single(const Operator &op);
 // The mesh-independent part of an operator: sizes, element numbers, D and
 // its even-odd tables, the domain faces of every element.
 int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
@@ -198,6 +202,8 @@ int vec_convert(T *a, const S *b, long n, cudaStream_t s);
 // w = mask(QQ^T A_L u + 0.1 u)  (ax, cg.f:96-125), unfused path.
 template <typename T>
 int apply_ax(const Operator &op, T *w, const T *u, const T *g, cudaStream_t s);
+// dssum on a device vector (dom as gs_exec)
+int dssum_dev(const Operator &op, void *u, int dom, cudaStream_t s);
 // the same in FP32 with the element products on the tensor cores (nb_ax_tc.cu)
 int apply_ax_tc(const Operator &op, float *w, const float *u, const float *g, cudaStream_t s);
 
