@@ -51,7 +51,8 @@ namespace {
 #define NB_BATCH_GROUP_CHUNK 2048
 #endif
 constexpr int kGroupChunk = NB_BATCH_GROUP_CHUNK;
-constexpr int kPointChunk = 2048;  // points per chunk, eight per thread
+// points per chunk at most, eight per thread: whole elements (at least one)
+constexpr int kPointChunk = 2048;
 constexpr int kThreads = 256;
 
 // ------------------------------------------------------------- kernels --
@@ -68,6 +69,16 @@ __global__ void __launch_bounds__(kThreads)
   const int ch = blockIdx.x;
   const int prob = gch_prob[ch];
   if (!sc[prob].active || !sc[prob].iactive) return;
+  if (sc[prob].box_ok) {  // the assembled update: only pap and alpha are left
+    const BatchProb P = pb[prob];
+    if (ch != P.gc0) return;
+    const double pap = block_sum_array(part_ax + P.el0, P.nelt, red);
+    if (threadIdx.x == 0) {
+      sc[prob].pap = pap;
+      sc[prob].alpha = pap != 0.0 ? sc[prob].rtz1 / pap : 0.0;
+    }
+    return;
+  }
   float part = 0.f;
   const int gend = gch_g0[ch + 1];
   for (int g = gch_g0[ch] + threadIdx.x; g < gend; g += kThreads) {
@@ -204,6 +215,27 @@ __global__ void k_bc_closed_form(const float *__restrict__ c, const int *__restr
   }
 }
 
+// Clears box_ok of every active problem whose residual differs (bitwise)
+// between copies of a point or is not zero where masked: its inner CG then takes the general iteration.
+// c32 verified beforehand (cf_ok), the mask is the full one.
+__global__ void __launch_bounds__(kThreads)
+    k_bcheck(const double *__restrict__ r, const int *__restrict__ off,
+             const unsigned *__restrict__ idx, const int *__restrict__ gch_g0,
+             const int *__restrict__ gch_prob, BatchScalars *sc) {
+  const int ch = blockIdx.x, prob = gch_prob[ch];
+  if (!sc[prob].active) return;
+  bool ok = true;
+  const int gend = gch_g0[ch + 1];
+  for (int g = gch_g0[ch] + threadIdx.x; g < gend; g += kThreads) {
+    const int b = off[g], e = off[g + 1];
+    const double v = r[idx[b] & 0x7fffffffu];
+    // (at a masked point the assembled form takes p = 0 for granted)
+    ok &= !(idx[b] & 0x80000000u) || (__double_as_longlong(v) << 1) == 0;
+    for (int q = b + 1; q < e; ++q) ok &= box_same(v, r[idx[q] & 0x7fffffffu]);
+  }
+  if (!__syncthreads_and(ok) && threadIdx.x == 0) sc[prob].box_ok = 0;
+}
+
 // The extreme-index bits of the points of one element of lx1 points a
 // direction, four points (one byte each: bit 0/1 i = 0 / lx1-1, 2/3 for j,
 // 4/5 for k) a word
@@ -243,8 +275,10 @@ __global__ void __launch_bounds__(kThreads)
            const BatchProb *__restrict__ pb, BatchScalars *sc, double *__restrict__ part_pt,
            unsigned *cnt, int it, int max_inner, double itol,
            const unsigned char *__restrict__ cface, const unsigned *__restrict__ ext4,
-           const float *__restrict__ pprev) {
+           const float *__restrict__ pprev, const unsigned char *__restrict__ cface_box,
+           const unsigned *__restrict__ bnd) {
   __shared__ double red[32];
+  __shared__ __align__(16) float wb[kPointChunk];
   const int ch = blockIdx.x;
   const int prob = pch_prob[ch];
   if (!sc[prob].active || !sc[prob].iactive) return;
@@ -257,7 +291,66 @@ __global__ void __launch_bounds__(kThreads)
                        reinterpret_cast<uintptr_t>(p) | reinterpret_cast<uintptr_t>(w) |
                        reinterpret_cast<uintptr_t>(c) |
                        (DEFER == 2 ? reinterpret_cast<uintptr_t>(pprev) : uintptr_t(0));
-  if ((al & 15u) == 0 && ((q0 | q1) & 3) == 0) {
+  if (sc[prob].box_ok) {
+    // the assembled update, as k_cg_update_box's FORM 2: the chunk's whole
+    // elements' boundary points first (the library's own vectors: aligned)
+    const BatchProb P = pb[prob];
+    const int lx = P.lx, l3 = lx * lx * lx, er = int((q0 - P.pt0) / l3), ne = int((q1 - q0) / l3);
+    BoxMesh box{};
+    box.nx = P.nelx;
+    box.ny = P.nely;
+    box.lx = lx;
+    const float *wp = w + P.pt0;
+    const unsigned char *fb0 = cface_box + P.el0 + er;
+    const int nf = 6 * (lx - 2) * (lx - 2), nr = P.nbnd - nf;
+#pragma unroll 3
+    for (int b = threadIdx.x; b < ne * nf; b += kThreads) {
+      const int el = ne > 1 ? b / nf : 0;
+      const unsigned u = __ldg(bnd + P.bnd0 + (b - el * nf)), nbr = __ldg(fb0 + el);
+      const int l = int(u & 0xFFFFu);
+      const unsigned ex = u >> 16;
+      const BoxCopies k = box_copies(box, (er + el) * l3 + l, ex & nbr);
+      const int d = k.d0 + k.d1 + k.d2;
+      const float a = wp[k.q0], o = wp[k.q0 + d];
+      wb[el * l3 + l] = (ex & ~nbr) ? 0.f : d ? add_rn(a, o) : a;
+    }
+    for (int b = threadIdx.x; b < ne * nr; b += kThreads) {
+      const int el = ne > 1 ? b / nr : 0;
+      const unsigned u = __ldg(bnd + P.bnd0 + nf + (b - el * nr)), nbr = __ldg(fb0 + el);
+      const int l = int(u & 0xFFFFu);
+      const unsigned ex = u >> 16;
+      float t = 0.f;
+      if (!(ex & ~nbr)) t = box_sum(wp, box_copies(box, (er + el) * l3 + l, ex & nbr));
+      wb[el * l3 + l] = t;
+    }
+    __syncthreads();
+    const int Q4 = l3 / 4, nv = int((q1 - q0) / 4);
+    for (int v = threadIdx.x; v < nv; v += kThreads) {
+      const int el = ne > 1 ? v / Q4 : 0;
+      const long gv = q0 / 4 + v;
+      alignas(16) float xa[4], pa[4], qa[4], ra[4], wa[4], ba[4];
+      if (DEFER != 1) {
+        *reinterpret_cast<float4 *>(xa) = reinterpret_cast<const float4 *>(x)[gv];
+        *reinterpret_cast<float4 *>(pa) = reinterpret_cast<const float4 *>(p)[gv];
+      }
+      if (DEFER == 2) *reinterpret_cast<float4 *>(qa) = reinterpret_cast<const float4 *>(pprev)[gv];
+      *reinterpret_cast<float4 *>(ra) = reinterpret_cast<const float4 *>(r)[gv];
+      *reinterpret_cast<float4 *>(wa) = reinterpret_cast<const float4 *>(w)[gv];
+      *reinterpret_cast<float4 *>(ba) = reinterpret_cast<const float4 *>(wb)[v];
+      const unsigned fb = __ldg(fb0 + el), b4 = __ldg(ext4 + P.ext0 + (v - el * Q4));
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const unsigned ex = (b4 >> (8 * q)) & 63u;
+        if (ex) wa[q] = ba[q];
+        if (DEFER == 2) xa[q] = fma_rn(alpha0, qa[q], xa[q]);
+        if (DEFER != 1) xa[q] = fma_rn(alpha, pa[q], xa[q]);
+        ra[q] = fma_rn(alphm, wa[q], ra[q]);
+        part = fma_rn(box_scale(ra[q], __popc(ex & fb)), ra[q], part);
+      }
+      if (DEFER != 1) reinterpret_cast<float4 *>(x)[gv] = *reinterpret_cast<const float4 *>(xa);
+      reinterpret_cast<float4 *>(r)[gv] = *reinterpret_cast<const float4 *>(ra);
+    }
+  } else if ((al & 15u) == 0 && ((q0 | q1) & 3) == 0) {
     // 16-byte accesses: chunk bounds are multiples of 4 (every lx1^3 of an
     // even lx1 is).  With cface: element le of the problem and group l4 of
     // v, advanced by the stride's quotient and remainder.
@@ -373,7 +466,7 @@ __global__ void __launch_bounds__(kThreads)
     k_bscale(float *__restrict__ r32, float *__restrict__ e32, const double *__restrict__ r,
              const float *__restrict__ c32, const long *__restrict__ pch_q0,
              const int *__restrict__ pch_prob, const BatchProb *__restrict__ pb,
-             BatchScalars *sc, double *__restrict__ part_pt, unsigned *cnt) {
+             BatchScalars *sc, double *__restrict__ part_pt, unsigned *cnt, int box) {
   __shared__ double red[32];
   const int ch = blockIdx.x;
   const int prob = pch_prob[ch];
@@ -399,6 +492,7 @@ __global__ void __launch_bounds__(kThreads)
       sc[prob].beta = 0.0;
       sc[prob].iactive = 1;
       sc[prob].pend = 0;
+      sc[prob].box_ok = box;  // (k_bcheck follows)
     }
   }
 }
@@ -651,6 +745,7 @@ struct Batch {
   // elements' face bits, the extreme-index tables of each lx1, one flag
   unsigned char *cface = nullptr;
   unsigned *ext4 = nullptr;
+  unsigned *bnd = nullptr;  // each lx1's boundary points (BoxMesh::bnd)
   int *cf_flag = nullptr;
   bool cf_ok = false;
   BatchScalars *sc = nullptr;
@@ -658,6 +753,9 @@ struct Batch {
   bool setup_done = false;
   // the solve graph
   cudaStream_t cap = nullptr;
+  std::vector<cudaStream_t> side;   // one per lx1 group but the first (each_group)
+  std::vector<cudaEvent_t> joined;
+  cudaEvent_t fork = nullptr;
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   double g_tol = -1.0, g_itol = -1.0;
@@ -668,13 +766,16 @@ struct Batch {
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     if (cap) cudaStreamDestroy(cap);
+    for (cudaStream_t t : side) cudaStreamDestroy(t);
+    for (cudaEvent_t e : joined) cudaEventDestroy(e);
+    if (fork) cudaEventDestroy(fork);
     for (auto &G : groups) {
       cudaFree(G.D64);
       cudaFree(G.D32);
     }
     void *ptrs[] = {x, f, g, c, r, w, g32, c32, r32, e32, p32, w32, el_prob, off, gch_g0,
                     gch_prob, pch_prob, cycles, idx, cnt, pch_q0, pb, sc, part_ax, part_gs,
-                    part_pt, cface, ext4, cf_flag, p32b};
+                    part_pt, cface, ext4, bnd, cf_flag, p32b};
     for (void *p : ptrs)
       if (p) cudaFree(p);
   }
@@ -686,8 +787,35 @@ struct Batch {
   bool paired() const { return g_paired_update && p32b; }
   float *dir(int it) const { return paired() && !(it & 1) ? p32b : p32; }
   float *dir_old(int it) const { return paired() && (it & 1) ? p32b : p32; }
+  // One launch per lx1 group, side by side: each group's own tail of blocks
+  // is filled by the others' (capture streams forked from s and joined).
+  template <typename F>
+  int each_group(cudaStream_t s, F launch) const {
+    if (groups.size() > 1) NB_CUDA(cudaEventRecord(fork, s));
+    for (size_t k = 0; k < groups.size(); ++k) {
+      const cudaStream_t t = k == 0 ? s : side[k - 1];
+      if (k > 0) NB_CUDA(cudaStreamWaitEvent(t, fork, 0));
+      NB_TRY(launch(groups[k], t));
+      if (k > 0) NB_CUDA(cudaEventRecord(joined[k - 1], t));
+    }
+    for (size_t k = 1; k < groups.size(); ++k) NB_CUDA(cudaStreamWaitEvent(s, joined[k - 1], 0));
+    return NB_OK;
+  }
+  int make_sides() {
+    if (groups.size() < 2 || fork) return NB_OK;
+    for (size_t k = 1; k < groups.size(); ++k) {
+      cudaStream_t t;
+      cudaEvent_t e;
+      NB_CUDA(cudaStreamCreateWithFlags(&t, cudaStreamNonBlocking));
+      side.push_back(t);
+      NB_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+      joined.push_back(e);
+    }
+    NB_CUDA(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    return NB_OK;
+  }
   int launch_inner_ax(int it, cudaStream_t s) const {
-    for (const auto &G : groups) {
+    return each_group(s, [&](const Group &G, cudaStream_t t) {
       BaxArgs<float> a{};
       a.w = w32;
       a.u = r32;
@@ -696,6 +824,7 @@ struct Batch {
       a.g = g32;
       a.c = c32;
       a.c_unit_interior = closed_c() ? 1 : 0;
+      a.cface = cf_ok ? cface : nullptr;
       a.D = G.D32;
       a.eo_h = G.EO.empty() ? nullptr : G.EO.data();
       a.el_prob = el_prob;
@@ -707,9 +836,8 @@ struct Batch {
       a.first = it == 1;
       a.err = device_error_word();
       a.wait_test = wait_test_mode();
-      NB_TRY(batch_ax_f32(G.lx, G.tune.epb32, G.tune.rd32, a, s));
-    }
-    return NB_OK;
+      return batch_ax_f32(G.lx, G.tune.epb32, G.tune.rd32, a, t);
+    });
   }
   // The FP64 defect's element operator for one group in shape epb64
   // (kFxShape: the fixed-point form after a separate x += |r| e).
@@ -766,8 +894,9 @@ struct Batch {
     return NB_OK;
   }
   int launch_defect_ax(cudaStream_t s) const {
-    for (const auto &G : groups) NB_TRY(defect_group_ax(G, G.tune.epb64, s));
-    return NB_OK;
+    return each_group(s, [&](const Group &G, cudaStream_t t) {
+      return defect_group_ax(G, G.tune.epb64, t);
+    });
   }
   static int batch_ax_f32(int lx, int epb, int rd, BaxArgs<float> a, cudaStream_t s) {
     if (!a.pold) a.pold = a.p;  // MODE 1 reads the old direction from pold
@@ -814,15 +943,15 @@ struct Batch {
     if (paired() && (it & 1) && it < max_inner)
       k_bupd<1><<<npc, kThreads, 0, s>>>(e32, r32, pc, w32, c32, pch_q0, pch_prob, pb, sc,
                                          part_pt, cnt + nprob, it, max_inner, itol, cf, ext4,
-                                         nullptr);
+                                         nullptr, cface, bnd);
     else if (paired() && !(it & 1))
       k_bupd<2><<<npc, kThreads, 0, s>>>(e32, r32, pc, w32, c32, pch_q0, pch_prob, pb, sc,
                                          part_pt, cnt + nprob, it, max_inner, itol, cf, ext4,
-                                         dir_old(it));
+                                         dir_old(it), cface, bnd);
     else
       k_bupd<0><<<npc, kThreads, 0, s>>>(e32, r32, pc, w32, c32, pch_q0, pch_prob, pb, sc,
                                          part_pt, cnt + nprob, it, max_inner, itol, cf, ext4,
-                                         nullptr);
+                                         nullptr, cface, bnd);
     NB_CUDA(cudaGetLastError());
     NB_TRY(mark(mk ? mk + 2 : nullptr, s));
     return NB_OK;
@@ -842,8 +971,12 @@ struct Batch {
   }
   int scale(cudaStream_t s) const {
     k_bscale<<<npc, kThreads, 0, s>>>(r32, e32, r, c32, pch_q0, pch_prob, pb, sc, part_pt,
-                                      cnt + 3 * nprob);
+                                      cnt + 3 * nprob, cf_ok ? 1 : 0);
     NB_CUDA(cudaGetLastError());
+    if (cf_ok) {
+      k_bcheck<<<ngc, kThreads, 0, s>>>(r, off, idx, gch_g0, gch_prob, sc);
+      NB_CUDA(cudaGetLastError());
+    }
     return NB_OK;
   }
   // initial norms, and the fixed-point metric of the solve (g may have
@@ -888,6 +1021,7 @@ struct Batch {
       o.ev.push_back(e);
     }
     if (!cap) NB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    NB_TRY(make_sides());
     NB_CUDA(cudaStreamBeginCapture(cap, cudaStreamCaptureModeRelaxed));
     int st = mark(&o.ev[0], cap);
     if (!st) st = scale(cap);
@@ -935,13 +1069,14 @@ struct Batch {
 
   int build_graph(double tol, int inner, int max_outer) {
     if (exec && tol == g_tol && inner == g_inner && max_outer == g_outer && itol == g_itol &&
-        wait_test_mode() == g_wtest && int(closed_c()) == g_cf && int(paired()) == g_pair)
+        wait_test_mode() == g_wtest && int(closed_c()) + 2 * int(cf_ok) == g_cf && int(paired()) == g_pair)
       return NB_OK;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
     exec = nullptr;
     graph = nullptr;
     if (!cap) NB_CUDA(cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking));
+    NB_TRY(make_sides());
     cudaGraph_t G = nullptr;
     NB_CUDA(cudaGraphCreate(&G, 0));
     graph = G;
@@ -1004,7 +1139,7 @@ struct Batch {
     g_outer = max_outer;
     g_itol = itol;
     g_wtest = wait_test_mode();
-    g_cf = int(closed_c());
+    g_cf = int(closed_c()) + 2 * int(cf_ok);
     g_pair = int(paired());
     return NB_OK;
   }
@@ -1068,10 +1203,10 @@ int batch_build(Batch *B, int nprob, const int *nx, const int *ny, const int *nz
   // concatenation
   B->P.resize(nprob);
   std::vector<int> el_prob, off_all, gch_g0, gch_prob, pch_prob;
-  std::vector<unsigned> idx_all, ext_all;
+  std::vector<unsigned> idx_all, ext_all, bnd_all;
   std::vector<long> pch_q0;
   long pt = 0;
-  int el = 0, gbase = 0, ext_lx0 = 0;
+  int el = 0, gbase = 0, ext_lx0 = 0, bnd_lx0 = 0;
   for (int s = 0; s < nprob; ++s) {
     const int p = order[s];
     const long l3 = long(lx[p]) * lx[p] * lx[p];
@@ -1088,8 +1223,15 @@ int batch_build(Batch *B, int nprob, const int *nx, const int *ny, const int *nz
       ext_lx0 = int(ext_all.size());
       const std::vector<unsigned> t = ext_table(lx[p]);
       ext_all.insert(ext_all.end(), t.begin(), t.end());
+      bnd_lx0 = int(bnd_all.size());
+      const std::vector<unsigned> bp = boundary_points(lx[p]);
+      bnd_all.insert(bnd_all.end(), bp.begin(), bp.end());
     }
     Q.ext0 = ext_lx0;
+    Q.nelx = nx[p];
+    Q.nely = ny[p];
+    Q.bnd0 = bnd_lx0;
+    Q.nbnd = int(bnd_all.size()) - bnd_lx0;
     for (long e = 0; e < nelt; ++e) el_prob.push_back(s);
     const int ngp = int(offs[s].size()) - 1;
     for (int q = 0; q < ngp; ++q)
@@ -1105,7 +1247,7 @@ int batch_build(Batch *B, int nprob, const int *nx, const int *ny, const int *nz
     }
     Q.ngc = int(gch_prob.size()) - Q.gc0;
     Q.pc0 = int(pch_prob.size());
-    for (long a = 0; a < Q.n; a += kPointChunk) {
+    for (long a = 0; a < Q.n; a += std::max(1L, kPointChunk / l3) * l3) {
       pch_q0.push_back(pt + a);
       pch_prob.push_back(s);
     }
@@ -1157,6 +1299,7 @@ int batch_build(Batch *B, int nprob, const int *nx, const int *ny, const int *nz
   NB_TRY(upload(&B->pch_prob, pch_prob));
   NB_TRY(upload(&B->pb, B->P));
   NB_TRY(upload(&B->ext4, ext_all));
+  NB_TRY(upload(&B->bnd, bnd_all));
   NB_TRY(dalloc(&B->cface, size_t(B->nelt)));
   NB_TRY(dalloc(&B->cf_flag, 1));
   NB_TRY(dalloc(&B->sc, nprob));

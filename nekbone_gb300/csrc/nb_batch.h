@@ -27,6 +27,8 @@ struct BatchScalars {
   int iactive;                               // 1 while the cycle's inner CG runs
   int pend;                                  // the inner CG stopped with its
                                              //   last x update deferred
+  int box_ok;                                // the cycle's inner CG takes the
+                                             //   assembled update (BoxMesh)
 };
 
 // Per-problem index ranges into the concatenated batch arrays.
@@ -37,6 +39,8 @@ struct BatchProb {
   int pc0, npc;     // point chunks
   int lx;           // points per direction
   int ext0;         // its lx1's extreme-index table in the batch's ext4
+  int nelx, nely;   // elements in x and y
+  int bnd0, nbnd;   // its lx1's boundary points (BoxMesh::bnd) in the batch's bnd
 };
 
 // Launch shape of the batched element operator for one lx1.
@@ -78,6 +82,8 @@ struct BaxArgs {
   int wait_test;       // timeout self-test of that wait (block_copy_begin)
   int c_unit_interior;  // MODE 1: c verified as the inverse multiplicity, so 1
                         //   at element-interior points: not read there
+  const unsigned char *cface;  // MODE 1: the elements' faces with a neighbour,
+                        //   for problems with box_ok (null: none has it)
 };
 
 // The batched element operator for one lx1 (T float: MODE 1, T double:

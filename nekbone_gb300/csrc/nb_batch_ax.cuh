@@ -171,6 +171,9 @@ __global__ void __launch_bounds__(LX * LX * EPB)
   }
 
   T part = T(0);
+  // the assembled update (BoxMesh): w' = w_L + 0.1 c p and pap at every point
+  const bool whole = MODE == 1 && a.cface && a.sc[prob].box_ok;
+  const unsigned nbr = whole ? a.cface[e] : 0u;
 #pragma unroll
   for (int k = 0; k < LX; ++k) {
     T tr, ts, tt;
@@ -198,7 +201,10 @@ __global__ void __launch_bounds__(LX * LX * EPB)
     const bool interior = col_interior && (k > 0) && (k < LX - 1);
     if (act) {
       if (MODE == 1) {
-        if (interior) {
+        if (whole) {
+          wl = fma_rn(box_tenth<T>(box_ext<LX>(i, j, k) & nbr), ureg[k], wl);
+          part = fma_rn(wl, ureg[k], part);
+        } else if (interior) {
           wl = fma_rn(T(0.1), ureg[k], wl);  // add2s2(w,u,.1,n), cg.f:119
           part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);
         }
@@ -287,6 +293,9 @@ __global__ void __launch_bounds__(LX * LX)
       pold[k] = T(a.e[id]);
     }
   }
+  // the assembled update (BoxMesh): w' = w_L + 0.1 c p and pap at every point
+  const bool whole = MODE == 1 && a.cface && a.sc[prob].box_ok;
+  const unsigned nbr = whole ? a.cface[e] : 0u;
 #pragma unroll
   for (int k = 0; k < LX; ++k) {
     const size_t id = base + size_t(k) * L2 + t;
@@ -367,7 +376,10 @@ __global__ void __launch_bounds__(LX * LX)
     const size_t id = base + size_t(k) * L2 + t;
     const bool interior = col_interior && (k > 0) && (k < LX - 1);
     if (MODE == 1) {
-      if (interior) {
+      if (whole) {
+        wl = fma_rn(box_tenth<T>(box_ext<LX>(i, j, k) & nbr), ureg[k], wl);
+        part = fma_rn(wl, ureg[k], part);
+      } else if (interior) {
         wl = fma_rn(T(0.1), ureg[k], wl);
         part = fma_rn(mul_rn(wl, creg[k]), ureg[k], part);
       }

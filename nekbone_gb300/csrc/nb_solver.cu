@@ -418,6 +418,21 @@ int operator_set_mask(Operator *op, const std::vector<int> &list_in) {
   return NB_OK;
 }
 
+std::vector<unsigned> boundary_points(int lx) {
+  std::vector<unsigned> of[64], pts;
+  for (int l = 0; l < lx * lx * lx; ++l) {
+    const int v[3] = {l % lx, (l / lx) % lx, l / (lx * lx)};
+    unsigned ex = 0;
+    for (int a = 0; a < 3; ++a)
+      ex |= (v[a] == 0 ? 1u : 0u) << (2 * a) | (v[a] == lx - 1 ? 1u : 0u) << (2 * a + 1);
+    if (ex) of[ex].push_back(unsigned(l) | ex << 16);
+  }
+  for (int kind = 1; kind <= 3; ++kind)
+    for (int f = 1; f < 64; ++f)
+      if (__builtin_popcount(f) == kind) pts.insert(pts.end(), of[f].begin(), of[f].end());
+  return pts;
+}
+
 int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
                   const int *lglel, const double *dxm1, int mask_mode, cudaStream_t s) {
   if (lx < 2 || lx > kMaxLx)
@@ -437,18 +452,7 @@ int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
   op->eo_ok = even_odd_tables(op->D, lx, op->EO);
   op->fx_ok = anti_centrosymmetric(op->D, lx) &&
               fx_tables(op->D, lx, op->FXhi, op->FXlo, op->FXd, &op->fx_fc);
-  // an element's boundary points, one face, edge or corner after the other
-  std::vector<unsigned> of[64], pts;
-  for (int l = 0; l < lx * lx * lx; ++l) {
-    const int v[3] = {l % lx, (l / lx) % lx, l / (lx * lx)};
-    unsigned ex = 0;
-    for (int a = 0; a < 3; ++a)
-      ex |= (v[a] == 0 ? 1u : 0u) << (2 * a) | (v[a] == lx - 1 ? 1u : 0u) << (2 * a + 1);
-    if (ex) of[ex].push_back(unsigned(l) | ex << 16);
-  }
-  for (int kind = 1; kind <= 3; ++kind)
-    for (int f = 1; f < 64; ++f)
-      if (__builtin_popcount(f) == kind) pts.insert(pts.end(), of[f].begin(), of[f].end());
+  const std::vector<unsigned> pts = boundary_points(lx);
   op->n_bnd_pts = int(pts.size());
   // one allocation: D in both precisions, these points, every point's bits,
   // room for element 0's mask, the elements' domain faces

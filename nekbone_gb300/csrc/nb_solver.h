@@ -144,6 +144,9 @@ int metric_fx_prepare(const Operator &op, const double *g, const double *D, cuda
 void metric_fx_invalidate(const Operator &op, bool solve);
 // The same before a single plain apply (apply_ax<double>, mode 0).
 void metric_fx_single(const Operator &op);
+// An element's boundary points, l | box_ext << 16, one face after the other,
+// then the edges, then the corners (BoxMesh::bnd).
+std::vector<unsigned> boundary_points(int lx);
 // The mesh-independent part of an operator: sizes, element numbers, D and
 // its even-odd tables, the domain faces of every element.
 int operator_base(Operator *op, int nelx, int nely, int nelz, int nelt, int lx,
