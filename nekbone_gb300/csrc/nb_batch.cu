@@ -721,6 +721,7 @@ struct Batch {
     // the fixed-point FP64 operator's tables and converted metric for this
     // group's elements (even lx1)
     std::shared_ptr<Operator> fx;
+    int uniform = 0;          // every FP32 metric block of the group is the same (setup)
     BatchTune tune;
   };
   int nprob = 0;
@@ -780,8 +781,17 @@ struct Batch {
       if (p) cudaFree(p);
   }
 
+  // one metric block a group where they are equal (not in the self-test of
+  // the bulk copies' waits, which would not be made)
+  bool shared_metric() const { return g_shared_metric && !wait_test_mode(); }
   // c formed in closed form by the inner iteration (verified at setup)
   bool closed_c() const { return cf_ok && g_mixed_closed_c; }
+  // what the graph's inner iteration was built for
+  int graph_key() const {
+    int k = int(closed_c()) + 2 * int(cf_ok) + 4 * int(shared_metric());
+    for (const auto &G : groups) k = 2 * k + G.uniform;
+    return k;
+  }
   // the inner CG's directions alternate between p32 (odd iterations) and
   // p32b (even), and x is updated once per pair (nb_set_paired_update)
   bool paired() const { return g_paired_update && p32b; }
@@ -825,6 +835,7 @@ struct Batch {
       a.c = c32;
       a.c_unit_interior = closed_c() ? 1 : 0;
       a.cface = cf_ok ? cface : nullptr;
+      a.g_uniform = shared_metric() && G.uniform;
       a.D = G.D32;
       a.eo_h = G.EO.empty() ? nullptr : G.EO.data();
       a.el_prob = el_prob;
@@ -1069,7 +1080,7 @@ struct Batch {
 
   int build_graph(double tol, int inner, int max_outer) {
     if (exec && tol == g_tol && inner == g_inner && max_outer == g_outer && itol == g_itol &&
-        wait_test_mode() == g_wtest && int(closed_c()) + 2 * int(cf_ok) == g_cf && int(paired()) == g_pair)
+        wait_test_mode() == g_wtest && graph_key() == g_cf && int(paired()) == g_pair)
       return NB_OK;
     if (exec) cudaGraphExecDestroy(exec);
     if (graph) cudaGraphDestroy(graph);
@@ -1139,7 +1150,7 @@ struct Batch {
     g_outer = max_outer;
     g_itol = itol;
     g_wtest = wait_test_mode();
-    g_cf = int(closed_c()) + 2 * int(cf_ok);
+    g_cf = graph_key();
     g_pair = int(paired());
     return NB_OK;
   }
@@ -1462,6 +1473,8 @@ int nb_batch_setup(nb_batch *b, uint64_t seed) {
   k_bc_closed_form<<<std::max(1, std::min(B.nelt, grid_for(long(B.nelt) * 256))), 256, 0, s>>>(
       B.c32, B.el_prob, B.pb, B.nelt, B.cface, B.cf_flag);
   NB_CUDA(cudaGetLastError());
+  for (auto &G : B.groups)
+    NB_TRY(metric_uniform(B.g32 + 6 * G.pt0, G.nel, G.lx, B.cycles, &G.uniform, s));
   int cf_h = 0;
   NB_CUDA(cudaMemcpyAsync(&cf_h, B.cf_flag, sizeof(int), cudaMemcpyDeviceToHost, s));
   // the fixed-point metric (allocated here, outside any graph capture;
@@ -1556,6 +1569,7 @@ int nb_batch_tune(nb_batch *b, int reps) {
       a.el0 = G.el0;
       a.nel = G.nel;
       a.first = 0;
+      a.g_uniform = B.shared_metric() && G.uniform;
       a.err = device_error_word();
       a.wait_test = wait_test_mode();
       st = Batch::batch_ax_f32(G.lx, sh.first, sh.second, a, s);

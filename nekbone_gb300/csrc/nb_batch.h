@@ -82,6 +82,8 @@ struct BaxArgs {
   int wait_test;       // timeout self-test of that wait (block_copy_begin)
   int c_unit_interior;  // MODE 1: c verified as the inverse multiplicity, so 1
                         //   at element-interior points: not read there
+  int g_uniform;       // every metric block of the group equals the first's: read that
+                        //   one (even-odd FP32 form)
   const unsigned char *cface;  // MODE 1: the elements' faces with a neighbour,
                         //   for problems with box_ok (null: none has it)
 };

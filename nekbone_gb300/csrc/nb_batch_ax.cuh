@@ -254,6 +254,7 @@ __global__ void __launch_bounds__(LX * LX)
   const int prob = a.el_prob[e];
   if (!a.sc[prob].active || (MODE == 1 && !a.sc[prob].iactive)) return;  // one element
   const size_t base = size_t(a.pt0) + size_t(blockIdx.x) * L3;
+  const T *gblk = a.g + 6 * (a.g_uniform ? size_t(a.pt0) : base);
   if (TMAG && t == 0)
     block_copy_begin(&sm.bar, sm.g, a.g + 6 * base, unsigned(6 * L3 * sizeof(T)), a.wait_test);
   // coefficients as in k_ax_eo: FP32 from the parameter bank, FP64 staged
@@ -329,10 +330,9 @@ __global__ void __launch_bounds__(LX * LX)
   for (int k = 0; k < LX; ++k) {
     const int q = eo_at<T, LX>(i, j, k);
     const T ur = sm.B[q], us = sm.C[q], ut = wtreg[k];
-    const size_t pt = base + size_t(k) * L2 + t;
     typedef typename Vec2<T>::type V2;
     const V2 *gp = TMAG ? reinterpret_cast<const V2 *>(&sm.g[6 * (k * L2 + t)])
-                        : reinterpret_cast<const V2 *>(a.g + 6 * pt);
+                        : reinterpret_cast<const V2 *>(gblk + 6 * (k * L2 + t));
     const V2 g01 = gp[0], g23 = gp[1], g45 = gp[2];
     T wr = mul_rn(g01.x, ur);
     wr = fma_rn(g01.y, us, wr);
@@ -398,12 +398,13 @@ __global__ void __launch_bounds__(LX * LX)
   if (t == 0) a.partial[e] = s;
 }
 
-template <typename T, int LX, int MODE>
+// TMAG: FP32's metric by bulk copy (element blocks are 16-byte aligned); without
+// it where one shared block serves the group.
+template <typename T, int LX, int MODE, bool TMAG>
 int launch_bax_eo(const BaxArgs<T> &a, cudaStream_t s) {
   if constexpr (LX % 2 != 0) {
     return fail(NB_ERR_UNSUPPORTED, "batched even-odd operator: odd lx1=%d", LX);
   } else {
-    constexpr bool TMAG = sizeof(T) == 4;   // element metric blocks are 16-byte aligned
     const size_t smem = sizeof(AxEoShared<T, LX, TMAG>);
     static bool attr = false;
     if (!attr) {
@@ -453,7 +454,9 @@ template <int LX>
 int batch_ax_f32_lx(int epb, int rd, const BaxArgs<float> &a, cudaStream_t s) {
   typedef BaxEpb<LX> P;
   if (rd == 2) {
-    if (epb == 1) return launch_bax_eo<float, LX, 1>(a, s);
+    if (epb == 1)
+      return a.g_uniform ? launch_bax_eo<float, LX, 1, false>(a, s)
+                         : launch_bax_eo<float, LX, 1, true>(a, s);
   } else if (rd) {
     if (epb == P::a) return launch_bax<float, LX, 1, true, P::a>(a, s);
     if (epb == P::b) return launch_bax<float, LX, 1, true, P::b>(a, s);
@@ -470,7 +473,7 @@ int batch_ax_f32_lx(int epb, int rd, const BaxArgs<float> &a, cudaStream_t s) {
 template <int LX>
 int batch_ax_f64_lx(int epb, const BaxArgs<double> &a, cudaStream_t s) {
   typedef BaxEpb<LX> P;
-  if (epb == 0) return launch_bax_eo<double, LX, 2>(a, s);   // even-odd form
+  if (epb == 0) return launch_bax_eo<double, LX, 2, false>(a, s);   // even-odd form
   if (epb == P::a) return launch_bax<double, LX, 2, false, P::a>(a, s);
   if (epb == P::b) return launch_bax<double, LX, 2, false, P::b>(a, s);
   return fail(NB_ERR_UNSUPPORTED, "batched FP64 operator: no shape epb=%d for lx1=%d", epb, LX);

@@ -224,7 +224,6 @@ int metric_uniform(const float *g32, long nelt, int lx, int *flag, int *uniform,
   const int one = 1;
   int h = 0;
   *uniform = 0;
-  if (!g_shared_metric) return NB_OK;
   NB_CUDA(cudaMemcpyAsync(flag, &one, sizeof(int), cudaMemcpyHostToDevice, s));
   if (nelt > 1) {
     const dim3 grid(unsigned((blk + 255) / 256), unsigned(std::min<long>(nelt - 1, 1024)));
@@ -277,7 +276,8 @@ int nb_cg_mixed(nb_mesh *mesh, double *x, const double *f, const double *g,
   int *flag = reinterpret_cast<int *>(wk.scratch + flags_at);
   unsigned char *cface = wk.scratch + flags_at + 16;
   bool closed = false;
-  if (!st) st = metric_uniform(g32, op.nelt, op.lx, flag, &uniform, s);
+  if (!st && g_shared_metric)
+    st = metric_uniform(g32, op.nelt, op.lx, flag, &uniform, s);
   if (!st && g_mixed_closed_c && op.fused_ok && !g_mixed_tc)
     st = c_closed_form(op, c32, cface, flag + 1, &closed, s);
   // x = 0, r = mask(f)

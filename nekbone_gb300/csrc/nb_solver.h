@@ -252,6 +252,11 @@ int time_cg_kernels_t(Operator &op, CgWork &wk, T *x, const T *f, const T *g,
 int cg_steps_pc(Operator &op, CgWork &wk, double *x, const double *g,
                 const double *c, double *r, double *w, double *p, double *z,
                 int it0, int it1, Precond *M, cudaStream_t s);
+// Whether every element of the FP32 metric g32 repeats element 0's block
+// (bitwise); synchronises s.  flag: one device int.
+int metric_uniform(const float *g32, long nelt, int lx, int *flag, int *uniform, cudaStream_t s);
+// nb_set_shared_metric: such a metric is read as one block (default true)
+extern bool g_shared_metric;
 // nb_set_mixed_closed_multiplicity: the inner FP32 CGs (single mesh and
 // batched) form c in closed form where it verifies (default true)
 extern bool g_mixed_closed_c;
