@@ -25,8 +25,12 @@ int launch_ax_eo_shape(AxArgs<T> a, const double *eo, cudaStream_t s) {
   }
   EoCoef<T, LX> cf;
   eo_fill(cf, eo);
-  fn<<<a.nelt, dim3(LX, LX), sm, s>>>(a, cf);
-  NB_CUDA(cudaGetLastError());
+  if constexpr (sizeof(T) == 4) {  // in a CG iteration, an apply
+    NB_CUDA(launch_dependent(fn, dim3(a.nelt), dim3(LX, LX), sm, s, a, cf));
+  } else {
+    fn<<<a.nelt, dim3(LX, LX), sm, s>>>(a, cf);
+    NB_CUDA(cudaGetLastError());
+  }
   return NB_OK;
 }
 

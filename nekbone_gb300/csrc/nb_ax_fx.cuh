@@ -800,6 +800,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
 template <int LX, int MODE>
 __global__ void __launch_bounds__((LX * LX + 31) / 32 * 32, (LX <= 12 ? NB_FX_MINB : 1))
     k_ax_fx(AxArgs<double> a, const __grid_constant__ FxCoef<LX> cf) {
+  dependent_begin();
   ax_fx_body<LX, MODE>(a, cf);
 }
 

@@ -27,8 +27,12 @@ int launch_ax_fx_shape(const Operator &op, AxArgs<double> a, cudaStream_t s) {
   }
   for (int q = 0; q < Coef::QD; ++q) cf.d[q] = Coef::FULL ? op.FXd[q] : 0;
   cf.fc = op.fx_fc;
-  fx::k_ax_fx<LX, MODE><<<a.nelt, dim3(LX, LX), sm, s>>>(a, cf);
-  NB_CUDA(cudaGetLastError());
+  if constexpr (MODE == 1 || MODE == 3) {  // in a CG iteration, an apply
+    NB_CUDA(launch_dependent(fx::k_ax_fx<LX, MODE>, dim3(a.nelt), dim3(LX, LX), sm, s, a, cf));
+  } else {
+    fx::k_ax_fx<LX, MODE><<<a.nelt, dim3(LX, LX), sm, s>>>(a, cf);
+    NB_CUDA(cudaGetLastError());
+  }
   return NB_OK;
 }
 

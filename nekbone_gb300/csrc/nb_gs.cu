@@ -13,7 +13,7 @@
 #include <float.h>
 #include <limits.h>
 
-#include "nb_internal.h"
+#include "nb_solver.h"
 
 namespace nb {
 
@@ -67,6 +67,7 @@ __device__ __forceinline__ T gs_identity() {
 template <typename T, int OP>
 __global__ void k_gs_sym(T *__restrict__ u, const int *__restrict__ off,
                          const int *__restrict__ idx, int ng) {
+  dependent_begin();
   for (int g = blockIdx.x * blockDim.x + threadIdx.x; g < ng; g += gridDim.x * blockDim.x) {
     const int b = off[g], e = off[g + 1];
     T t = u[idx[b]];
@@ -164,7 +165,8 @@ void run_gs(const GsDevice &d, T *u, int transpose, cudaStream_t s) {
   const int TB = 256;
   if (d.symmetric) {
     if (d.ng > 0)
-      k_gs_sym<T, OP><<<sym_grid<T, OP>(d.ng), TB, 0, s>>>(u, d.off, d.idx, d.ng);
+      launch_dependent(k_gs_sym<T, OP>, dim3(sym_grid<T, OP>(d.ng)), dim3(TB), 0, s, u, d.off,
+                       d.idx, d.ng);
     return;
   }
   const int *og = transpose ? d.off_s : d.off_g, *ig = transpose ? d.idx_s : d.idx_g;

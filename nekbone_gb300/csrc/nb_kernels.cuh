@@ -41,6 +41,19 @@ __device__ __forceinline__ double uniform_pm1(uint64_t seed, uint64_t id) {
   return double(z >> 11) * (2.0 / 9007199254740992.0) - 1.0;
 }
 
+// ---------------------------------------------------- dependent launches --
+// First statement of the kernels of a CG iteration and of an apply.  They are
+// launched with programmatic stream serialisation (launch_dependent): the
+// launch is set up while the kernel before still runs, and the blocks wait
+// here until it has finished and its writes are visible.  50 CG iterations
+// (three kernels each) on 4^3 elements, lx1 = 10: 1.39 -> 1.03 ms; 16^3
+// deformed, lx1 = 8: 5.05 -> 4.65 ms.  Letting the next kernel's blocks in
+// early as well (launch_dependents at the start) took that back: 1.45 ms, and
+// 83 instead of 69 ms at 32^3, lx1 = 12.  Launched plainly, it does nothing.
+__device__ __forceinline__ void dependent_begin() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // ------------------------------------------------------------ reduction --
 // Deterministic block sum of one value per thread: a fixed shuffle tree in
 // the accumulation type A (float for the FP32 kernels, which keeps FP64
@@ -555,6 +568,7 @@ __global__ void __launch_bounds__(256, NB_GS_MINB)
              int n_ax_partial, unsigned *counter, CgScalars *sc, const BoxMesh box,
              const int *box_ok) {
   __shared__ double red[32];
+  dependent_begin();
   if (box_flag(box_ok)) {  // the assembled update: only pap and alpha are left
     box_alpha(w, p, partial, ax_partial, n_ax_partial, counter, sc, box, red);
     return;
@@ -696,6 +710,7 @@ __global__ void __launch_bounds__(256)
                 double *hist, int iter, int identity_precond,
                 float *__restrict__ r32 = nullptr, const T *__restrict__ pprev = nullptr,
                 const unsigned char *__restrict__ cface = nullptr, int lx = 0) {
+  dependent_begin();
   __shared__ double red[32];
   // CF: the extreme-index bits of the four points of each 16-byte group
   // of an element, one byte a point
@@ -859,6 +874,7 @@ __global__ void __launch_bounds__(256, 8)
   extern __shared__ __align__(128) unsigned char smem_raw[];
   __shared__ double red[32];
   struct alignas(VEC * sizeof(T)) Pack { T v[VEC]; };
+  dependent_begin();
   const bool whole = sc->box_ok != 0;
   const int lx = box.lx, l3 = lx * lx * lx, ne = FORM == 2 ? ne_ : 1;
   const T alpha = T(sc->alpha);
@@ -1074,6 +1090,7 @@ __global__ void __launch_bounds__(256)
     k_box_assemble(T *__restrict__ w, const T *__restrict__ u, const BoxMesh box,
                    unsigned total) {
   const unsigned l3 = unsigned(box.lx * box.lx * box.lx);
+  dependent_begin();
 #pragma unroll 2
   for (unsigned v = blockIdx.x * blockDim.x + threadIdx.x; v < total;
        v += gridDim.x * blockDim.x) {
@@ -1148,6 +1165,7 @@ __global__ void __launch_bounds__(256)
             unsigned *counter, double *out, CgScalars *sc, int mode,
             double *hist, int iter, const float *__restrict__ mf = nullptr,
             T *mout = nullptr) {
+  dependent_begin();
   __shared__ double red[32];
   T part = T(0);
   // 16-byte accesses (two doubles or four floats a thread) when every vector
@@ -1488,6 +1506,7 @@ __device__ __forceinline__ void ax_eo_body(const AxArgs<T> &a, const EoCoef<T, L
 template <typename T, int LX, int MODE, bool TMAG>
 __global__ void __launch_bounds__(LX * LX)
     k_ax_eo(AxArgs<T> a, const __grid_constant__ EoCoef<T, LX> cf) {
+  dependent_begin();
   ax_eo_body<T, LX, MODE, TMAG>(a, cf);
 }
 // The same with four CTAs per SM asked for (the FP64 lx1 = 12 operator):

@@ -123,6 +123,7 @@ inline int line_grid(int n, int nelt) { return grid_for(long(n) * n * nelt); }
 // element's own layer-2 value, ghost edges and corners zero.
 template <typename T>
 __global__ void k_toext(T *A, const T *r, int nh, int nelt) {
+  dependent_begin();
   const int nl = nh + 2, nl2 = nl * nl, nh2 = nh * nh, hi = nl - 1;
   const int lines = nl2 * nelt;
   // ghost coordinate 0 reads layer 2, nl-1 reads layer nl-3 (regular index - 1)
@@ -166,6 +167,7 @@ __device__ __forceinline__ T ghost_minus_at(const T *Ae, int a, int b, int c, in
 // hsmg.f:1084: A <- 0*A + B on the ghost faces).
 template <typename T>
 __global__ void k_fdm(T *B, T *A, const T *s, const T *d, int nl) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *sm = reinterpret_cast<T *>(sm_raw);
   const int nl2 = nl * nl, nl3 = nl2 * nl;
@@ -276,6 +278,7 @@ __device__ __forceinline__ void fdm_tensor3(T *X, T *Y, const T *C3) {
 template <typename T, int NL>
 __global__ void __launch_bounds__(FdmShape<T, NL>::THREADS)
     k_fdm_fixed(T *B, T *A, const T *s, const T *d) {
+  dependent_begin();
   typedef FdmShape<T, NL> F;
   constexpr int NL2 = F::NL2, NL3 = F::NL3, PS = F::PS, IP = F::IP, MS = NL * IP, HI = NL - 1;
   extern __shared__ __align__(16) unsigned char sm_raw[];
@@ -395,10 +398,10 @@ int launch_fdm(T *B, T *A, const T *s, const T *d, int nl, int nelt, cudaStream_
     size_t sm;
     int th;
     fdm_fixed_shape<T>(nl, &sm, &th);
-    fn<<<nelt, th, sm, st>>>(B, A, s, d);
+    NB_CUDA(launch_dependent(fn, dim3(nelt), dim3(th), sm, st, B, A, s, d));
+  } else {
+    NB_CUDA(launch_dependent(k_fdm<T>, dim3(nelt), dim3(256), fdm_smem<T>(nl), st, B, A, s, d, nl));
   }
-  else k_fdm<T><<<nelt, 256, fdm_smem<T>(nl), st>>>(B, A, s, d, nl);
-  NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
 
@@ -408,6 +411,7 @@ int launch_fdm(T *B, T *A, const T *s, const T *d, int nl, int nelt, cudaStream_
 // layer-2 partner it is.
 template <typename T>
 __global__ void k_overlap_toreg(T *e_out, const T *B, const T *A, int nh, int nelt) {
+  dependent_begin();
   const int nl = nh + 2, nl2 = nl * nl, nh2 = nh * nh, lines = nh2 * nelt;
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < lines; t += gridDim.x * blockDim.x) {
     const int e = t / nh2, ab = t - e * nh2, a = ab % nh + 1, b = ab / nh + 1;
@@ -466,6 +470,7 @@ __device__ __forceinline__ T schwarz_weigh(T x, const T *we, int n, int i, int j
 template <typename T>
 __global__ void k_rstr(T *v, const T *u, const T *wt, int nu, int nv, const T *jht,
                        const T *jh) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *sm = reinterpret_cast<T *>(sm_raw);
   const int nu3 = nu * nu * nu, nmax = max(nu, nv), nmax3 = nmax * nmax * nmax;
@@ -499,6 +504,7 @@ __global__ void k_rstr(T *v, const T *u, const T *wt, int nu, int nv, const T *j
 template <typename T>
 __global__ void k_intp_add(T *out, const T *uc, int nu, int nv, const T *jh, const T *jht,
                            const T *wt) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *sm = reinterpret_cast<T *>(sm_raw);
   const int nmax = max(nu, nv), nmax3 = nmax * nmax * nmax;
@@ -588,6 +594,7 @@ constexpr size_t xfer_smem() {
 template <typename T, int NU, int NV>
 __global__ void __launch_bounds__(256) k_rstr_fixed(T *v, const T *u, const T *wt,
                                                     const T *jht, const T *jh) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *us = reinterpret_cast<T *>(sm_raw), *work = us + NU * NU * NU, *work2 = work + NV * NU * NU,
     *Jt = work2 + NV * NV * NU, *J = Jt + NU * NV;
@@ -617,6 +624,7 @@ __global__ void __launch_bounds__(256) k_rstr_fixed(T *v, const T *u, const T *w
 template <typename T, int NU, int NV>
 __global__ void __launch_bounds__(256) k_intp_fixed(T *out, const T *uc, const T *jh,
                                                     const T *jht, const T *wt) {
+  dependent_begin();
   extern __shared__ __align__(16) unsigned char sm_raw[];
   T *us = reinterpret_cast<T *>(sm_raw), *work = us + NU * NU * NU, *work2 = work + NV * NU * NU,
     *J = work2 + NV * NV * NU, *Jt = J + NU * NV;
@@ -873,6 +881,7 @@ int overlap_sum(const MgLevel &L, int nelt, double *e, double *B, double *A,
 }  // namespace
 
 __global__ void k_to_f32(float *y, const double *x, long n) {
+  dependent_begin();
   for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
        q += long(gridDim.x) * blockDim.x)
     y[q] = float(x[q]);
@@ -1214,11 +1223,13 @@ int mg_schwarz(Multigrid &mg, T *e, T *r, int l, T *A, T *B, bool mask_r, cudaSt
   MgLevel &L = mg.lv[l];
   const int nelt = mg.op->nelt;
   if (mask_r) NB_TRY(vec_mask<T>(r, L.mask, L.nmask, s));
-  k_toext<T><<<line_grid(L.nl, nelt), 256, 0, s>>>(A, r, L.nh, nelt);
+  NB_CUDA(launch_dependent(k_toext<T>, dim3(line_grid(L.nl, nelt)), dim3(256), 0, s, A,
+                           (const T *)r, L.nh, nelt));
   NB_TRY(gs_exec(L.gsx, A, V::dom, 1, 0, s));
   NB_TRY(launch_fdm<T>(B, A, V::fast_s(L), V::fast_d(L), L.nl, nelt, s));
   NB_TRY(gs_exec(L.gsx, B, V::dom, 1, 0, s));
-  k_overlap_toreg<T><<<line_grid(L.nh, nelt), 256, 0, s>>>(e, B, A, L.nh, nelt);
+  NB_CUDA(launch_dependent(k_overlap_toreg<T>, dim3(line_grid(L.nh, nelt)), dim3(256), 0, s, e,
+                           (const T *)B, (const T *)A, L.nh, nelt));
   NB_TRY(gs_exec(L.gs, e, V::dom, 1, 0, s));
   NB_TRY(vec_mask<T>(e, L.mask, L.nmask, s));
   NB_CUDA(cudaGetLastError());
@@ -1231,7 +1242,8 @@ int mg_rstr(Multigrid &mg, T *rc, const T *rf, int l, bool dssum, cudaStream_t s
   const MgLevel &F = mg.lv[l + 1], &C = mg.lv[l];
   const XferFixed<T> fx = xfer_fixed<T>(F.nh, C.nh);
   if (fx.rstr) {
-    fx.rstr<<<mg.op->nelt, 256, fx.smem_rstr, s>>>(rc, rf, V::rstr_wt(F), V::jht(C), V::jh(C));
+    NB_CUDA(launch_dependent(fx.rstr, dim3(mg.op->nelt), dim3(256), fx.smem_rstr, s, rc, rf,
+                             V::rstr_wt(F), V::jht(C), V::jh(C)));
   } else {
     const int nmax = std::max(F.nh, C.nh);
     k_rstr<T><<<mg.op->nelt, 256, tensor_smem(nmax, 2 * F.nh * C.nh) * sizeof(T) / 8, s>>>(
@@ -1251,7 +1263,8 @@ int mg_intp_add(Multigrid &mg, T *of, const T *ec, int l, bool weigh, cudaStream
   const T *wt = weigh ? V::schwarz_wt(F) : nullptr;
   const XferFixed<T> fx = xfer_fixed<T>(F.nh, C.nh);
   if (fx.intp) {
-    fx.intp<<<mg.op->nelt, 256, fx.smem_intp, s>>>(of, ec, V::jh(C), V::jht(C), wt);
+    NB_CUDA(launch_dependent(fx.intp, dim3(mg.op->nelt), dim3(256), fx.smem_intp, s, of, ec,
+                             V::jh(C), V::jht(C), wt));
   } else {
     const int nmax = std::max(F.nh, C.nh);
     k_intp_add<T><<<mg.op->nelt, 256, tensor_smem(nmax, 2 * F.nh * C.nh) * sizeof(T) / 8, s>>>(
@@ -1262,6 +1275,7 @@ int mg_intp_add(Multigrid &mg, T *of, const T *ec, int l, bool weigh, cudaStream
 }
 
 __global__ void k_to_f64(double *y, const float *x, long n) {
+  dependent_begin();
   for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < n;
        q += long(gridDim.x) * blockDim.x)
     y[q] = double(x[q]);
@@ -1270,11 +1284,13 @@ __global__ void k_to_f64(double *y, const float *x, long n) {
 // ---- exact coarse solve ----------------------------------------------------
 // b(i) = assembled residual at coarse vertex i (its first copy after dssum)
 __global__ void k_coarse_gather(double *b, const double *e1, const int *prim, int nc) {
+  dependent_begin();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < nc) b[i] = e1[prim[i]];
 }
 // e1(q) = x(gid(q)), 0 at masked points
 __global__ void k_coarse_scatter(double *e1, const double *x, const int *gid, long n1) {
+  dependent_begin();
   for (long q = long(blockIdx.x) * blockDim.x + threadIdx.x; q < n1;
        q += long(gridDim.x) * blockDim.x) {
     const int c = gid[q];
@@ -1285,6 +1301,7 @@ __global__ void k_coarse_scatter(double *e1, const double *x, const int *gid, lo
 // sums in a fixed order, then a fixed shuffle tree
 __global__ void __launch_bounds__(256) k_dense_mv(double *y, const double *A,
                                                   const double *x, int n) {
+  dependent_begin();
   const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   if (warp >= n) return;

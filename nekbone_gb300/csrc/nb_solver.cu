@@ -555,6 +555,7 @@ __global__ void k_convert(T *a, const S *b, long n) {
 }
 template <typename T>
 __global__ void k_mask_list(T *w, const int *list, int nlist) {
+  dependent_begin();
   const int q = blockIdx.x * blockDim.x + threadIdx.x;
   if (q < nlist) w[list[q]] = T(0);
 }
@@ -669,9 +670,8 @@ void update_box_launch(const Operator &op, const CgWork &wk, T *x, T *r, const T
   }
   const long units = FORM == 0 ? (op.n + nt - 1) / nt : (op.nelt + ne - 1) / ne;
   const int grid = int(std::min<long>(std::min(wk.grid_up, resident[op.lx]), units));
-  k_cg_update_box<T, D, VEC, FORM><<<grid, nt, sm, s>>>(x, r, p, w, c, op.n, wk.partial_up,
-                                                        wk.counters + 1, wk.sc, hist, iter,
-                                                        pprev, wk.box, ne);
+  launch_dependent(k_cg_update_box<T, D, VEC, FORM>, dim3(grid), dim3(nt), sm, s, x, r, p, w, c,
+                   op.n, wk.partial_up, wk.counters + 1, wk.sc, hist, iter, pprev, wk.box, ne);
 }
 
 // The third kernel of an iteration, pairing mode D: the assembled update on
@@ -698,15 +698,15 @@ void update_launch(const Operator &op, const CgWork &wk, T *x, T *r, const T *p,
   }
   if constexpr (std::is_same<T, float>::value) {
     if (wk.c32_face) {
-      k_cg_update<T, D, true><<<wk.grid_up, 256, 0, s>>>(
-          x, r, p, w, c, op.n, wk.partial_up, wk.counters + 1, wk.sc, hist, iter, identity,
-          r32, pprev, wk.c32_face, op.lx);
+      launch_dependent(k_cg_update<T, D, true>, dim3(wk.grid_up), dim3(256), 0, s, x, r, p, w, c,
+                       op.n, wk.partial_up, wk.counters + 1, wk.sc, hist, iter, identity, r32,
+                       pprev, wk.c32_face, op.lx);
       return;
     }
   }
-  k_cg_update<T, D><<<wk.grid_up, 256, 0, s>>>(x, r, p, w, c, op.n, wk.partial_up,
-                                               wk.counters + 1, wk.sc, hist, iter, identity,
-                                               r32, pprev);
+  launch_dependent(k_cg_update<T, D, false>, dim3(wk.grid_up), dim3(256), 0, s, x, r, p, w, c,
+                   op.n, wk.partial_up, wk.counters + 1, wk.sc, hist, iter, identity, r32, pprev,
+                   (const unsigned char *)nullptr, 0);
 }
 }  // namespace
 
@@ -725,8 +725,8 @@ int vec_add2s2(T *a, const T *b, double c1, long n, cudaStream_t s) {
 template <typename T>
 int vec_mask(T *w, const int *list, int nlist, cudaStream_t s) {
   if (nlist <= 0) return NB_OK;
-  k_mask_list<T><<<(nlist + 255) / 256, 256, 0, s>>>(w, list, nlist);
-  NB_CUDA(cudaGetLastError());
+  NB_CUDA(launch_dependent(k_mask_list<T>, dim3((nlist + 255) / 256), dim3(256), 0, s, w, list,
+                           nlist));
   return NB_OK;
 }
 template <typename T>
@@ -745,9 +745,8 @@ int vec_glsc3(const T *a, const T *b, const T *m, long n, CgWork &wk,
               double *out, CgScalars *sc, int mode, int iter, cudaStream_t s,
               const float *mf, T *mout) {
   const int gr = std::min(grid_for(n), wk.grid_up);
-  k_glsc3<T><<<gr, 256, 0, s>>>(a, b, m, n, wk.partial_dot, wk.counters + 2, out,
-                                sc, mode, wk.hist, iter, mf, mout);
-  NB_CUDA(cudaGetLastError());
+  NB_CUDA(launch_dependent(k_glsc3<T>, dim3(gr), dim3(256), 0, s, a, b, m, n, wk.partial_dot,
+                           wk.counters + 2, out, sc, mode, wk.hist, iter, mf, mout));
   return NB_OK;
 }
 
@@ -800,8 +799,8 @@ static int box_assemble(const Operator &op, const BoxMesh &b, T *w, const T *u, 
   }
   const long total = long(op.nelt) * b.nbnd;  // below n
   const int grid = int(std::max(1L, std::min<long>(resident, (total + 255) / 256)));
-  k_box_assemble<T, AX><<<grid, 256, 0, s>>>(w, u, b, unsigned(total));
-  NB_CUDA(cudaGetLastError());
+  NB_CUDA(launch_dependent(k_box_assemble<T, AX>, dim3(grid), dim3(256), 0, s, w, u, b,
+                           unsigned(total)));
   return NB_OK;
 }
 
@@ -942,11 +941,9 @@ static int cg_steps_t(Operator &op, CgWork &wk, T *x, const T *g, const T *c,
       a.box = wk.box;
       a.box_ok = box_ok(wk);
       NB_TRY(launch_ax<T>(op, 1, a, s));
-      k_gs_fin<T><<<wk.grid_gs, 256, 0, s>>>(w, p, c, op.bnd_off, op.bnd_idx,
-                                             op.nbg, wk.partial_gs, wk.partial_ax,
-                                             op.nelt, wk.counters + 0, wk.sc, wk.box,
-                                             box_ok(wk));
-      NB_CUDA(cudaGetLastError());
+      NB_CUDA(launch_dependent(k_gs_fin<T>, dim3(wk.grid_gs), dim3(256), 0, s, w, p, c,
+                               op.bnd_off, op.bnd_idx, op.nbg, wk.partial_gs, wk.partial_ax,
+                               op.nelt, wk.counters + 0, wk.sc, wk.box, box_ok(wk)));
     } else {
       if (iter == 1)
         k_copy_first<T><<<grid_for(n), 256, 0, s>>>(p, zz, n);

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <memory>
+#include <utility>
 #include <vector>
 
 #include "nb_internal.h"
@@ -177,6 +178,23 @@ int operator_set_mask(Operator *op, const std::vector<int> &list);
 std::vector<int> full_mask_list(const Operator &op);
 
 // ------------------------------------------------------------- kernels --
+// A launch on s that may start before the one before it has finished: for
+// kernels that begin with dependent_begin().
+template <typename... P, typename... A>
+cudaError_t launch_dependent(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             A &&...args) {
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = &at;
+  c.numAttrs = 1;
+  return cudaLaunchKernelEx(&c, k, std::forward<A>(args)...);
+}
 template <typename T>
 int launch_ax(const Operator &op, int mode, AxArgs<T> a, cudaStream_t s);
 template <>
