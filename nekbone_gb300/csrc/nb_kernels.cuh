@@ -1076,19 +1076,74 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The boundary points of a box in place, in closed form: t = sum of w over the
-// copies in jl's order, then every copy gets t (AX false: dssum,
-// prox_dssum.f:2-12) or t + 0.1 u, 0 when masked (AX: the rest of ax,
-// cg.f:117-120, after an operator with `tenth`).  A thread takes a point's
-// lowest copy; the boundary points come kind by kind (BoxMesh::bnd), so a
-// warp's threads mostly do the same, and whole warps skip the faces whose
-// points have a lower copy.  Bound by the latency of its gathers, as the
-// group lists' pass: ax at 16^3, lx1 = 12 in FP64 31 us, where the
-// gather-scatter, add2s2 and mask passes took 25 + 23 + 4.
-template <typename T, bool AX>
+// dssum (prox_dssum.f:2-12) on a box in place, in closed form: every copy of a
+// boundary point gets the sum over the copies in jl's order.  A thread takes a
+// point's lowest copy: first the points inside the elements' upper faces (i, j
+// or k = lx1-1), a pair of copies each and four points in flight a thread,
+// then the edges and corners.  Bound by the latency of its gathers; no index
+// lists.  24 x 20 x 22 elements, lx1 = 10, FP64: 36 us, 41 with the groups'
+// lists or with one point in flight.
+template <typename T>
+__global__ void __launch_bounds__(256) k_box_dssum(T *__restrict__ w, const BoxMesh box, int nelt) {
+  const unsigned l3 = unsigned(box.lx * box.lx * box.lx);
+  const unsigned nfc = unsigned((box.lx - 2) * (box.lx - 2)), nr = unsigned(box.nbnd) - 6u * nfc;
+  const unsigned v0 = blockIdx.x * blockDim.x + threadIdx.x, vs = gridDim.x * blockDim.x;
+  dependent_begin();
+  constexpr int K = 4;
+  const unsigned n1 = unsigned(nelt) * 3u * nfc;
+  for (unsigned v = v0; v < n1; v += K * vs) {
+    int q[K], d[K];
+    T a[K], o[K];
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      const unsigned vk = v + k * vs;
+      d[k] = 0;
+      if (vk >= n1) continue;
+      const unsigned e = vk / (3u * nfc), b = vk - e * 3u * nfc, f = b / nfc;
+      const unsigned en = __ldg(box.bnd + ((2u * f + 1u) * nfc + (b - f * nfc)));
+      const unsigned cp = (en >> 16) & box_neighbours(box, int(e));
+      if (!cp) continue;
+      q[k] = int(e * l3 + (en & 0xFFFFu));
+      const BoxCopies c = box_copies(box, 0, cp);
+      d[k] = c.d0 + c.d1 + c.d2;
+      a[k] = w[q[k]];
+      o[k] = w[q[k] + d[k]];
+    }
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (!d[k]) continue;
+      const T t = add_rn(a[k], o[k]);
+      w[q[k]] = t;
+      w[q[k] + d[k]] = t;
+    }
+  }
+  const unsigned n2 = unsigned(nelt) * nr;
+  for (unsigned v = v0; v < n2; v += vs) {
+    const unsigned e = v / nr, b = v - e * nr;
+    const unsigned en = __ldg(box.bnd + 6u * nfc + b);
+    const unsigned cp = (en >> 16) & box_neighbours(box, int(e));
+    if ((cp & 21u) || !cp) continue;  // a lower copy's, or alone
+    const int q = int(e * l3 + (en & 0xFFFFu));
+    const BoxCopies k = box_copies(box, q, cp);
+    const T t = box_sum(w, k);
+#pragma unroll
+    for (int m = 0; m < 8; ++m) {
+      if (((m & 1) && !k.d0) || ((m & 2) && !k.d1) || ((m & 4) && !k.d2)) continue;
+      w[q + (m & 1 ? k.d0 : 0) + (m & 2 ? k.d1 : 0) + (m & 4 ? k.d2 : 0)] = t;
+    }
+  }
+}
+
+// The rest of ax on a box (cg.f:117-120), after an operator with `tenth`: the
+// boundary points' sums over the copies + 0.1 u, 0 when masked.  A thread
+// takes a point's lowest copy; the boundary points come kind by kind
+// (BoxMesh::bnd), so a warp's threads mostly do the same, and whole warps skip
+// the faces whose points have a lower copy.  ax at 16^3, lx1 = 12 in FP64:
+// 31 us, where the gather-scatter, add2s2 and mask passes took 25 + 23 + 4
+// (with k_box_dssum's four points in flight 40 us, at 63 registers).
+template <typename T>
 __global__ void __launch_bounds__(256)
-    k_box_assemble(T *__restrict__ w, const T *__restrict__ u, const BoxMesh box,
-                   unsigned total) {
+    k_box_rest(T *__restrict__ w, const T *__restrict__ u, const BoxMesh box, unsigned total) {
   const unsigned l3 = unsigned(box.lx * box.lx * box.lx);
   dependent_begin();
 #pragma unroll 2
@@ -1097,21 +1152,17 @@ __global__ void __launch_bounds__(256)
     const unsigned e = v / unsigned(box.nbnd), b = v - e * unsigned(box.nbnd);
     const unsigned en = __ldg(box.bnd + b), ex = en >> 16, nbr = box_neighbours(box, int(e));
     const unsigned cp = ex & nbr;
-    if ((cp & 21u) || (!AX && !cp)) continue;  // a lower copy's, or alone
+    if (cp & 21u) continue;  // a lower copy's
     const int q = int(e * l3 + (en & 0xFFFFu));
     const BoxCopies k = box_copies(box, q, cp);
     const T t = box_sum(w, k);
-    const bool all = AX && box.full_mask && (ex & ~nbr) != 0u;
-    const bool own = AX && !box.full_mask && e == 0u && box.mask0[en & 0xFFFFu] != 0;
-    const unsigned have = (k.d0 ? 2u : 0u) | (k.d1 ? 4u : 0u) | (k.d2 ? 16u : 0u);
+    const bool all = box.full_mask && (ex & ~nbr) != 0u;
+    const bool own = !box.full_mask && e == 0u && box.mask0[en & 0xFFFFu] != 0;
 #pragma unroll
     for (int m = 0; m < 8; ++m) {
-      const unsigned need = (m & 1 ? 2u : 0u) | (m & 2 ? 4u : 0u) | (m & 4 ? 16u : 0u);
-      if (need & ~have) continue;
+      if (((m & 1) && !k.d0) || ((m & 2) && !k.d1) || ((m & 4) && !k.d2)) continue;
       const int id = q + (m & 1 ? k.d0 : 0) + (m & 2 ? k.d1 : 0) + (m & 4 ? k.d2 : 0);
-      T r = t;
-      if (AX) r = all || (own && m == 0) ? T(0) : fma_rn(T(0.1), u[id], t);
-      w[id] = r;
+      w[id] = all || (own && m == 0) ? T(0) : fma_rn(T(0.1), u[id], t);
     }
   }
 }

@@ -788,28 +788,39 @@ static int maskit_dev(Operator &op, T *w, cudaStream_t s) {
   return vec_mask<T>(w, op.d_mask_list, op.n_mask, s);
 }
 
-// the boundary points of a box in place (k_box_assemble)
-template <typename T, bool AX>
-static int box_assemble(const Operator &op, const BoxMesh &b, T *w, const T *u, cudaStream_t s) {
-  static int resident = 0;
-  if (!resident) {
-    int k = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_box_assemble<T, AX>, 256, 0);
-    resident = sm_count() * std::max(1, k);
-  }
+// the resident blocks of a kernel of 256 threads: the most a grid-stride pass
+// is launched with
+template <typename K>
+static int resident_256(K kernel) {
+  int k = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kernel, 256, 0);
+  return sm_count() * std::max(1, k);
+}
+static int stride_grid(long items, int resident) {
+  return int(std::max(1L, std::min<long>(resident, (items + 255) / 256)));
+}
+
+template <typename T>
+static int box_dssum(const Operator &op, const BoxMesh &b, T *w, cudaStream_t s) {
+  static const int resident = resident_256(k_box_dssum<T>);
+  const int grid = stride_grid(long(op.nelt) * b.nbnd / 2, resident);
+  NB_CUDA(launch_dependent(k_box_dssum<T>, dim3(grid), dim3(256), 0, s, w, b, op.nelt));
+  return NB_OK;
+}
+
+template <typename T>
+static int box_rest(const Operator &op, const BoxMesh &b, T *w, const T *u, cudaStream_t s) {
+  static const int resident = resident_256(k_box_rest<T>);
   const long total = long(op.nelt) * b.nbnd;  // below n
-  const int grid = int(std::max(1L, std::min<long>(resident, (total + 255) / 256)));
-  NB_CUDA(launch_dependent(k_box_assemble<T, AX>, dim3(grid), dim3(256), 0, s, w, u, b,
-                           unsigned(total)));
+  NB_CUDA(launch_dependent(k_box_rest<T>, dim3(stride_grid(total, resident)), dim3(256), 0, s, w,
+                           u, b, unsigned(total)));
   return NB_OK;
 }
 
 int dssum_dev(const Operator &op, void *u, int dom, cudaStream_t s) {
   const BoxMesh b = op.box_shape();
-  if (b.nx > 0 && dom == 1)
-    return box_assemble<double, false>(op, b, static_cast<double *>(u), nullptr, s);
-  if (b.nx > 0 && dom == 2)
-    return box_assemble<float, false>(op, b, static_cast<float *>(u), nullptr, s);
+  if (b.nx > 0 && dom == 1) return box_dssum<double>(op, b, static_cast<double *>(u), s);
+  if (b.nx > 0 && dom == 2) return box_dssum<float>(op, b, static_cast<float *>(u), s);
   return gs_exec(op.gs, u, dom, 1, 0, s);
 }
 
@@ -827,7 +838,7 @@ int apply_ax(const Operator &op_c, T *w, const T *u, const T *g, cudaStream_t s)
   NB_TRY(launch_ax<T>(op, 0, a, s));
   if (a.tenth) {
     const BoxMesh b = op.box_mesh();
-    if (b.nx > 0) return box_assemble<T, true>(op, b, w, u, s);
+    if (b.nx > 0) return box_rest<T>(op, b, w, u, s);
     k_ax_rest<T><<<grid_for(op.nbg), 256, 0, s>>>(w, u, op.bnd_off, op.bnd_idx, op.nbg);
     NB_CUDA(cudaGetLastError());
     return NB_OK;

@@ -1,4 +1,4 @@
-"""The closed-form assembly of a box's boundary points (k_box_assemble)
+"""The closed-form assembly of a box's boundary points (k_box_dssum, k_box_rest)
 against jl's gather-scatter on the same numbering: dssum bitwise in both
 precisions, and the operator's second pass through a numbering in another
 element order (the boundary groups instead) against the oracle."""
