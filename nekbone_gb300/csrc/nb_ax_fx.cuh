@@ -316,8 +316,8 @@ struct FxShared {
   i64 A[N];
   i64 C[N];
   i64 D[N];
-  int emax[8], gmax[8];
-  unsigned orl[8], orh[8];
+  int emax[24], gmax[24];
+  unsigned orl[24], orh[24];
   double red[32];
 };
 
@@ -793,6 +793,155 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     const double s = block_sum<double>(part, sm.red);
     if (t == 0) a.partial[e] = s;
   }
+}
+
+// The CG pass (MODE 1) with three threads a column instead of one, for meshes
+// too small to fill the SMs: thread (grp, i, j) takes the lines of direction
+// grp in the contraction stages and a third of the column's points elsewhere,
+// so an element takes a third of the time (and fewer elements fit an SM).  The
+// same values as ax_fx_body and ax_sep_body at every point; pap's partial sums
+// in another order.  ax_fx_is_wide says where, with both forms measured.
+template <int LX>
+__device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef<LX> &cf) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  FxShared<LX> &sm = *reinterpret_cast<FxShared<LX> *>(smem_raw);
+  constexpr int L2 = LX * LX, L3 = LX * LX * LX, NTH = 3 * L2, NW = (NTH + 31) / 32;
+  constexpr int BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 2 : 0, NK = (LX + 2) / 3;
+  constexpr bool SEP = !FxCoef<LX>::FULL;
+  const int tid = threadIdx.x, grp = tid / L2, t = tid - grp * L2, i = t % LX, j = t / LX;
+  const int e = blockIdx.x, w = tid >> 5, k0 = grp * NK;
+  const size_t base = size_t(e) * L3;
+  const bool whole = box_flag(a.box_ok);
+  const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
+  const int2 sep = SEP && a.sep ? *reinterpret_cast<const int2 *>(a.sep) : make_int2(0, 0);
+  if (SEP && sep.x && tid < FxShared<LX>::NT) sm.tab[tid] = a.sep->tab[tid];
+  const unsigned lanes = warp_mask(NTH, w);
+  int em = 0;
+  {
+    double uk[NK], pold[NK];
+    const double beta = !a.first ? a.sc->beta : 0.0;
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {  // all loads before the first store
+      uk[q] = pold[q] = 0.0;
+      if (k0 + q >= LX) break;
+      const size_t id = base + size_t(k0 + q) * L2 + t;
+      uk[q] = a.u[id];
+      if (!a.first) pold[q] = a.pold[id];
+    }
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {
+      if (k0 + q >= LX) break;
+      if (!a.first) uk[q] = fma_rn(beta, pold[q], uk[q]);  // add2s1, math.f:534
+      a.p[base + size_t(k0 + q) * L2 + t] = uk[q];
+      em = max(em, bexp(uk[q]));
+    }
+    const int r = __reduce_max_sync(lanes, unsigned(em));
+    if ((tid & 31) == 0) sm.emax[w] = r;
+    __syncthreads();
+    em = 0;
+    for (int q = 0; q < NW; ++q) em = max(em, sm.emax[q]);
+#pragma unroll
+    for (int q = 0; q < NK; ++q) {
+      if (k0 + q >= LX) break;
+      sm.A[fx_at<LX>(i, j, k0 + q)] =
+          SEP && sep.x ? to_fixed60(uk[q], em) : to_fixed_cvt(uk[q], em, BITS - 53);
+    }
+  }
+  __syncthreads();
+
+  // the group's lines: along i (j, k), along j (i, k), along k (i, j)
+  const int b0 = grp == 0 ? fx_at<LX>(0, j, i) : grp == 1 ? fx_at<LX>(i, 0, j) : fx_at<LX>(i, j, 0);
+  const int st = grp == 0 ? 1 : grp == 1 ? LX : (LX * LX + 1);
+  i64 *out = grp == 0 ? sm.A : grp == 1 ? sm.C : sm.D;
+  i64 v[LX];
+#pragma unroll
+  for (int m = 0; m < LX; ++m) v[m] = sm.A[b0 + m * st];
+  __syncthreads();  // every line of A is read
+  double part = 0.0;
+  bool done = false;
+  if constexpr (SEP) {
+    if (sep.x) {
+      fx_line_sep<LX>(v, sm.tab, [&](int m, i64 y) { out[b0 + m * st] = y; });
+      __syncthreads();
+      const int sY = em - 1075 - (60 - 53) + 64 - sep.y;
+      const bool bad = em == 0x7FF;
+      auto wloc = [&](int k) {
+        const int q = fx_at<LX>(i, j, k);
+        return mul_rn(to_double_cvt(sm.A[q] + sm.C[q] + sm.D[q], sY),
+                      __ldg(a.sep->v + k * L2 + t));
+      };
+      part = whole ? ax_fx_finish<LX, 1, NK, true>(a, e, t, k0, bad, nbr, wloc)
+                   : ax_fx_finish<LX, 1, NK, false>(a, e, t, k0, bad, nbr, wloc);
+      done = true;
+    }
+  }
+  if (!done) {
+    u64 orv = 0;
+    fx_line<LX>(v, cf, 0, [&](int m, i64 y) {
+      out[b0 + m * st] = y;
+      orv |= mag(y);
+    });
+    fx_or_post(orv, sm.orl, sm.orh, tid, NTH);
+    __syncthreads();
+    int s1 = fx_or_shift(sm.orl, sm.orh, NTH, BITS);
+    if (s1 < 0) {  // outside the bounds shift_up relies on: results invalid
+      if (tid == 0 && a.err) atomicOr(a.err, 2u);
+      s1 = 0;
+    }
+    const int eg = a.gexp[e];
+    const int sW = 64 - MK + (eg - 1082) + (em - 1075 - (BITS - 53)) - cf.fc + 64 - s1;
+    __syncthreads();  // orl, orh are written again below
+    orv = 0;
+#pragma unroll
+    for (int k_ = 0; k_ < NK; ++k_) {
+      const int k = k0 + k_;
+      if (k >= LX) break;
+      const int q = fx_at<LX>(i, j, k);
+      const Sp ur = split(shift_up(sm.A[q], s1)), us = split(shift_up(sm.C[q], s1)),
+               ut = split(shift_up(sm.D[q], s1));
+      const int4 *gp = reinterpret_cast<const int4 *>(a.gfx + 6 * (base + size_t(k) * L2 + t));
+      const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
+      const Sp G1 = {g01.x, g01.y}, G2 = {g01.z, g01.w}, G3 = {g23.x, g23.y},
+               G4 = {g23.z, g23.w}, G5 = {g45.x, g45.y}, G6 = {g45.z, g45.w};
+      Acc<MK> wr, ws, wt;
+      wr.mac(G1, ur); wr.mac(G2, us); wr.mac(G3, ut);
+      ws.mac(G2, ur); ws.mac(G4, us); ws.mac(G5, ut);
+      wt.mac(G3, ur); wt.mac(G5, us); wt.mac(G6, ut);
+      const i64 r_ = wr.result(), s_ = ws.result(), t_ = wt.result();
+      sm.A[q] = r_;
+      sm.C[q] = s_;
+      sm.D[q] = t_;
+      orv |= mag(r_) | mag(s_) | mag(t_);
+    }
+    fx_or_post(orv, sm.orl, sm.orh, tid, NTH);
+    __syncthreads();
+    int s2 = fx_or_shift(sm.orl, sm.orh, NTH, BITS);
+    if (s2 < 0) {  // as s1
+      if (tid == 0 && a.err) atomicOr(a.err, 2u);
+      s2 = 0;
+    }
+    const int sT = 64 - cf.fc + sW - s2;
+#pragma unroll
+    for (int m = 0; m < LX; ++m) v[m] = shift_up(out[b0 + m * st], s2);
+    fx_line<LX>(v, cf, 1, [&](int m, i64 y) { out[b0 + m * st] = y; });
+    __syncthreads();
+    const bool bad = em == 0x7FF || eg == 0x7FF;
+    auto wloc = [&](int k) {
+      const int q = fx_at<LX>(i, j, k);
+      return to_double_cvt(sm.A[q] + sm.C[q] + sm.D[q], sT);
+    };
+    part = whole ? ax_fx_finish<LX, 1, NK, true>(a, e, t, k0, bad, nbr, wloc)
+                 : ax_fx_finish<LX, 1, NK, false>(a, e, t, k0, bad, nbr, wloc);
+  }
+  const double s = block_sum<double>(part, sm.red);
+  if (tid == 0) a.partial[e] = s;
+}
+
+template <int LX>
+__global__ void __launch_bounds__((3 * LX * LX + 31) / 32 * 32)
+    k_ax_fx_wide(AxArgs<double> a, const __grid_constant__ FxCoef<LX> cf) {
+  dependent_begin();
+  ax_fx_wide<LX>(a, cf);
 }
 
 // (the thread bound is the whole warps the block occupies, so that the
