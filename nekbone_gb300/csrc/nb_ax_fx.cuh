@@ -317,7 +317,9 @@ struct FxShared {
   i64 C[N];
   i64 D[N];
   int emax[24], gmax[24];
-  unsigned orl[24], orh[24];
+  // one pair for each of the two renormalisations (fx_or_post): a warp may
+  // post the second while another still reads the first
+  unsigned orl[2][24], orh[2][24];
   double red[32];
 };
 
@@ -704,9 +706,9 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
       orv |= mag(y);
     });
   }
-  fx_or_post(orv, sm.orl, sm.orh, t, L2);
+  fx_or_post(orv, sm.orl[0], sm.orh[0], t, L2);
   __syncthreads();
-  int s1 = fx_or_shift(sm.orl, sm.orh, L2, BITS);
+  int s1 = fx_or_shift(sm.orl[0], sm.orh[0], L2, BITS);
   if (s1 < 0) {  // outside the bounds shift_up relies on: results invalid
     if (t == 0 && a.err) atomicOr(a.err, 2u);
     s1 = 0;
@@ -754,9 +756,9 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     sm.D[q] = t_;
     orv |= mag(r_) | mag(s_) | mag(t_);
   }
-  fx_or_post(orv, sm.orl, sm.orh, t, L2);
+  fx_or_post(orv, sm.orl[1], sm.orh[1], t, L2);
   __syncthreads();
-  int s2 = fx_or_shift(sm.orl, sm.orh, L2, BITS);
+  int s2 = fx_or_shift(sm.orl[1], sm.orh[1], L2, BITS);
   if (s2 < 0) {  // as s1
     if (t == 0 && a.err) atomicOr(a.err, 2u);
     s2 = 0;
@@ -881,16 +883,15 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
       out[b0 + m * st] = y;
       orv |= mag(y);
     });
-    fx_or_post(orv, sm.orl, sm.orh, tid, NTH);
+    fx_or_post(orv, sm.orl[0], sm.orh[0], tid, NTH);
     __syncthreads();
-    int s1 = fx_or_shift(sm.orl, sm.orh, NTH, BITS);
+    int s1 = fx_or_shift(sm.orl[0], sm.orh[0], NTH, BITS);
     if (s1 < 0) {  // outside the bounds shift_up relies on: results invalid
       if (tid == 0 && a.err) atomicOr(a.err, 2u);
       s1 = 0;
     }
     const int eg = a.gexp[e];
     const int sW = 64 - MK + (eg - 1082) + (em - 1075 - (BITS - 53)) - cf.fc + 64 - s1;
-    __syncthreads();  // orl, orh are written again below
     orv = 0;
 #pragma unroll
     for (int k_ = 0; k_ < NK; ++k_) {
@@ -913,9 +914,9 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
       sm.D[q] = t_;
       orv |= mag(r_) | mag(s_) | mag(t_);
     }
-    fx_or_post(orv, sm.orl, sm.orh, tid, NTH);
+    fx_or_post(orv, sm.orl[1], sm.orh[1], tid, NTH);
     __syncthreads();
-    int s2 = fx_or_shift(sm.orl, sm.orh, NTH, BITS);
+    int s2 = fx_or_shift(sm.orl[1], sm.orh[1], NTH, BITS);
     if (s2 < 0) {  // as s1
       if (tid == 0 && a.err) atomicOr(a.err, 2u);
       s2 = 0;
