@@ -1021,8 +1021,9 @@ __global__ void __launch_bounds__(256, 8)
 
 // The start of a solve on a box (cg.f:36-42): x = 0, r = mask(f), rnorm, and
 // whether the assembled update holds (BoxMesh); sc->box_ok is set before and
-// cleared here.  f may be r itself.  One pass instead of a memset, a copy, a
-// mask and a glsc3.
+// cleared here.  f may be r itself (then only masked points are written: the
+// others' copies are read meanwhile); x null: it is zero already.  One pass
+// instead of a memset, a copy, a mask and a glsc3.
 template <typename T>
 __global__ void __launch_bounds__(256)
     k_box_begin(T *x, const T *f, T *r, const T *c, long n, double *__restrict__ partial,
@@ -1049,7 +1050,7 @@ __global__ void __launch_bounds__(256)
       if (cp & 32u) ok &= box_same(fv, f[q + d.d2]);
     }
     if (x) x[q] = T(0);
-    r[q] = rv;
+    if (f != r || masked) r[q] = rv;
     part = fma_rn(mul_rn(rv, cv), rv, part);
     l += sl;
     e += se;

@@ -873,6 +873,7 @@ static int cg_begin_t(Operator &op, CgWork &wk, T *x, const T *f, const T *c,
   if (std::is_same<T, double>::value) metric_fx_invalidate(op, op.fused_ok && !unfused);
   // the reference's list is built by its first mask (of r, below)
   const bool built = op.mask_built || op.mask_mode == 1;
+  T *x0 = x;  // (f and r may be the same vector)
   if (!built || !plain || !box_form<T>(op)) {
     NB_CUDA(cudaMemsetAsync(x, 0, n * sizeof(T), s));  // rzero(x)
     NB_TRY(vec_copy<T>(r, f, n, s));                   // copy(r,f)
@@ -880,11 +881,12 @@ static int cg_begin_t(Operator &op, CgWork &wk, T *x, const T *f, const T *c,
     if (!plain || !box_form<T>(op))
       return vec_glsc3<T>(r, c, r, n, wk, wk.dot_out, wk.sc, 1, 0, s);
     f = r;
+    x0 = nullptr;  // both done
   }
   wk.box = op.box_mesh();
   NB_CUDA(cudaMemsetAsync(&wk.sc->box_ok, 1, sizeof(int), s));
-  k_box_begin<T><<<wk.grid_up, 256, 0, s>>>(f == r ? nullptr : x, f, r, c, n, wk.partial_up,
-                                            wk.counters + 1, wk.sc, wk.hist, wk.box);
+  k_box_begin<T><<<wk.grid_up, 256, 0, s>>>(x0, f, r, c, n, wk.partial_up, wk.counters + 1,
+                                            wk.sc, wk.hist, wk.box);
   NB_CUDA(cudaGetLastError());
   return NB_OK;
 }
