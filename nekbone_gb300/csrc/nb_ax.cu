@@ -29,12 +29,10 @@ int launch_ax<double>(const Operator &op, int mode, AxArgs<double> a, cudaStream
     // a single apply (metric_fx_single) converts the metric as it goes
     if (mode == 0 && op.metric_single && (reinterpret_cast<uintptr_t>(a.g) & 15u) == 0)
       return launch_ax_fx_m3(op, a, s);
-    NB_TRY(metric_fx_prepare(op, a.g, op.dD, s));
+    NB_TRY(metric_fx_prepare(op, a.g, op.dD, mode != 0, s));
     a.gfx = op.gfx;
     a.gexp = op.gexp;
     a.sep = op.sep_on ? op.sep : nullptr;
-    if (mode == 0 && a.sep)
-      return fail(NB_ERR_STATE, "ax: a plain apply inside a solve on the separable metric");
     if (mode == 0) return launch_ax_fx_m0(op, a, s);
     if (mode == 1) return launch_ax_fx_m1(op, a, s);
     return launch_ax_fx_m2(op, a, s);

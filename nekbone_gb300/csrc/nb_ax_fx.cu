@@ -289,18 +289,19 @@ bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
   return ok;
 }
 
-void metric_fx_invalidate(const Operator &op, bool solve) {
+void metric_fx_invalidate(const Operator &op) {
   op.gfx_src = nullptr;
-  op.metric_solve = solve;
   op.metric_single = false;
 }
 void metric_fx_single(const Operator &op) {
-  metric_fx_invalidate(op, false);
+  metric_fx_invalidate(op);
   op.metric_single = true;
 }
 
-int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s) {
-  if (op.gfx_src == g && op.gfx) return NB_OK;
+int metric_fx_prepare(const Operator &op, const double *g, const double *D, bool fused,
+                      cudaStream_t s) {
+  // (plain applies after fused ones have no separable form to go by)
+  if (op.gfx_src == g && op.gfx && (fused || !op.sep_on)) return NB_OK;
   const long nv = 6 * op.n;
   if (op.gfx_cap < nv) {
     if (op.gfx) cudaFree(op.gfx);
@@ -317,7 +318,7 @@ int metric_fx_prepare(const Operator &op, const double *g, const double *D, cuda
   }
   const int blk = 6 * op.lx * op.lx * op.lx;
   // the separable form's check pays from the second apply on
-  const bool sep = op.metric_solve && op.lx % 2 == 0;
+  const bool sep = fused && op.lx % 2 == 0;
   op.sep_on = sep;
   if (sep) {
     NB_CUDA(cudaMemsetAsync(&op.sep->ok, 1, sizeof(int), s));

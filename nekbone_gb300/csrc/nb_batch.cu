@@ -899,8 +899,8 @@ struct Batch {
   int convert_metric(cudaStream_t s) const {
     for (const auto &G : groups)
       if (G.fx && G.tune.epb64 == kFxShape) {
-        metric_fx_invalidate(*G.fx, true);
-        NB_TRY(metric_fx_prepare(*G.fx, g + 6 * G.pt0, G.D64, s));
+        metric_fx_invalidate(*G.fx);
+        NB_TRY(metric_fx_prepare(*G.fx, g + 6 * G.pt0, G.D64, true, s));
       }
     return NB_OK;
   }
@@ -1481,8 +1481,8 @@ int nb_batch_setup(nb_batch *b, uint64_t seed) {
   // every solve converts it again)
   for (auto &G : B.groups)
     if (G.fx) {
-      metric_fx_invalidate(*G.fx, true);
-      NB_TRY(metric_fx_prepare(*G.fx, B.g + 6 * G.pt0, G.D64, s));
+      metric_fx_invalidate(*G.fx);
+      NB_TRY(metric_fx_prepare(*G.fx, B.g + 6 * G.pt0, G.D64, true, s));
     }
   NB_CUDA(cudaStreamSynchronize(s));
   B.cf_ok = cf_h != 0;

@@ -259,7 +259,7 @@ int nb_cg_mixed(nb_mesh *mesh, double *x, const double *f, const double *g,
   // r, w (FP64); g32 (6n), c32, r32, e32, rr32, w32, p32, p32b (FP32); two
   // int flags; the elements' face bits (nelt bytes)
   int st = wk.ensure(op, std::max(inner_iters, 1));
-  metric_fx_invalidate(op, op.fused_ok);
+  metric_fx_invalidate(op);
   const size_t flags_at = size_t(n) * (2 * 8 + 13 * 4);
   if (!st) st = wk.ensure_scratch(flags_at + 16 + size_t(op.nelt));
   if (st) return st;

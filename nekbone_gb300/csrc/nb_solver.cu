@@ -861,16 +861,15 @@ static bool box_form(const Operator &op) {
 }
 
 // cg.f:36-42: x = 0, r = mask(f), rnorm = sqrt(glsc3(r,c,r)).  plain: the
-// solve runs the fused iteration without preconditioner; unfused: it runs the
-// unfused one by request.
+// solve runs the fused iteration without preconditioner.
 template <typename T>
 static int cg_begin_t(Operator &op, CgWork &wk, T *x, const T *f, const T *c,
-                      T *r, bool plain, int niter, cudaStream_t s, bool unfused = false) {
+                      T *r, bool plain, int niter, cudaStream_t s) {
   const long n = op.n;
   NB_TRY(wk.ensure(op, niter));
   wk.r32_ready = false;
   wk.box = BoxMesh{};
-  if (std::is_same<T, double>::value) metric_fx_invalidate(op, op.fused_ok && !unfused);
+  if (std::is_same<T, double>::value) metric_fx_invalidate(op);
   // the reference's list is built by its first mask (of r, below)
   const bool built = op.mask_built || op.mask_mode == 1;
   T *x0 = x;  // (f and r may be the same vector)
@@ -1117,7 +1116,7 @@ int cg_device(Operator &op, CgWork &wk, double *x, const double *f,
               const double *g, const double *c, double *r, double *w,
               double *p, double *z, int niter, Precond *M, bool force_unfused,
               cudaStream_t s) {
-  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, !M && !force_unfused, niter, s, force_unfused));
+  NB_TRY(cg_begin_t<double>(op, wk, x, f, c, r, !M && !force_unfused, niter, s));
   // the second direction buffer of the paired x update (fused, no
   // preconditioner, at least one pair)
   double *p_alt = nullptr;

@@ -36,7 +36,6 @@ struct Operator {
   mutable int *gexp = nullptr;
   mutable fx::SepTables *sep = nullptr;  // its separable form (even lx only),
   mutable bool sep_on = false;           //   looked for in this solve
-  mutable bool metric_solve = false;
   mutable bool metric_single = false;    // one plain apply: no conversion pass
   mutable const double *gfx_src = nullptr;
   mutable long gfx_cap = 0;
@@ -137,12 +136,13 @@ bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
 // The metric g in the fixed-point operator's form, converted when g is not
 // the array last converted: the separable form where g has it (op.sep),
 // else op.gfx / op.gexp (one pass over g each, decided on the device);
-// metric_fx_invalidate forgets
-// the conversion (every solve and every standalone apply starts with it, so
-// a caller may change g's contents between calls); solve: several fused
-// applies (modes 1 and 2) follow, and the separable form is looked for.
-int metric_fx_prepare(const Operator &op, const double *g, const double *D, cudaStream_t s);
-void metric_fx_invalidate(const Operator &op, bool solve);
+// metric_fx_invalidate forgets the conversion (every solve and every standalone
+// apply starts with it, so a caller may change g's contents between calls).
+// fused: for fused applies (modes 1 and 2), of which several follow: the
+// separable form is looked for.  Plain applies (mode 0) take the general form.
+int metric_fx_prepare(const Operator &op, const double *g, const double *D, bool fused,
+                      cudaStream_t s);
+void metric_fx_invalidate(const Operator &op);
 // The same before a single plain apply (apply_ax<double>, mode 0).
 void metric_fx_single(const Operator &op);
 // An element's boundary points, l | box_ext << 16, one face after the other,
