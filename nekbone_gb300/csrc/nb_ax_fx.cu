@@ -54,11 +54,11 @@ int64_t scaled_sum(const double *x, int nx, int sh) {
 }
 
 // one block per element: the element's largest exponent over its 6 lx1^3
-// metric values, then each value as balanced halves of g 2^(1082 - emax)
+// metric values, then each value as balanced halves of g 2^(1022 + bits - emax)
 // (nothing where the separable form holds)
 __global__ void __launch_bounds__(256)
     k_metric_fx(const double *__restrict__ g, int2 *__restrict__ gfx, int *__restrict__ gexp,
-                int blk, const fx::SepTables *sep) {
+                int blk, int bits, const fx::SepTables *sep) {
   __shared__ int wmax[8];
   if (sep && sep->ok) return;
   const int t = threadIdx.x;
@@ -71,7 +71,7 @@ __global__ void __launch_bounds__(256)
   em = 0;
   for (int w = 0; w < 8; ++w) em = max(em, wmax[w]);
   for (int q = t; q < blk; q += 256) {
-    const fx::Sp s = fx::split(fx::to_fixed(g[base + q], em, 7));
+    const fx::Sp s = fx::split(fx::to_fixed(g[base + q], em, bits - 53));
     gfx[base + q] = make_int2(s.lo, s.hi);
   }
   if (t == 0) gexp[blockIdx.x] = em;
@@ -217,8 +217,8 @@ __global__ void __launch_bounds__(256)
 // bits.
 bool fx_tables(const std::vector<double> &D, int lx, std::vector<int> &hi,
                std::vector<int> &lo, std::vector<int> &d, int *fc) {
-  // lx1 = 13 and 15 keep the reference's FP64 sums: on random fields this
-  // form's error there is 1.1 to 1.5 times theirs (up to 11 it is smaller)
+  // lx1 = 13 and 15 keep the reference's FP64 sums: on random fields one apply
+  // of this form has 1.1 to 1.5 times their error there (up to 11 less than it)
   if (lx < 2 || (lx % 2 != 0 && lx > 11)) return false;
   const int h = lx / 2, h1 = lx - h;
   const bool full = h1 > h;
@@ -324,7 +324,8 @@ int metric_fx_prepare(const Operator &op, const double *g, const double *D, bool
     NB_CUDA(cudaMemsetAsync(&op.sep->ok, 1, sizeof(int), s));
     k_sep_check<<<std::min(op.nelt, 152 * 8), 256, 0, s>>>(g, D, op.lx, op.nelt, op.sep);
   }
-  k_metric_fx<<<op.nelt, 256, 0, s>>>(g, op.gfx, op.gexp, blk, sep ? op.sep : nullptr);
+  k_metric_fx<<<op.nelt, 256, 0, s>>>(g, op.gfx, op.gexp, blk, fx::fx_gbits(op.lx),
+                                       sep ? op.sep : nullptr);
   NB_CUDA(cudaGetLastError());
   op.gfx_src = g;
   return NB_OK;

@@ -92,9 +92,10 @@ __device__ __forceinline__ Sp split(i64 x) {
 // of half the length), x started at half a unit so that the high word of
 // x + x2 rounds to nearest (al*bl dropped).  Each product is one 32x32 ->
 // 64-bit multiply-add (mad.wide.s32), written in C++ so that a coefficient
-// can stay a constant-bank operand.  For the three terms of the metric step;
-// K = 2 keeps two more bits of its outputs.
-template <int K>
+// can stay a constant-bank operand.  For the three terms of the metric step.
+// The FULL form (FxCoef) takes K = 3, three more bits of its outputs, and the
+// high word of al*bl (|x + x2| <= 6 * 2^60 for |c|, |v| <= 2^61).
+template <int K, bool FULL = false>
 struct Acc {
   i64 hh, x, x2;
   __device__ __forceinline__ Acc() : hh(0), x(1ll << (31 - K)), x2(0) {}
@@ -102,6 +103,7 @@ struct Acc {
     hh += i64(c.hi) * i64(v.hi);
     x += i64(c.hi) * i64(v.lo);
     x2 += i64(c.lo) * i64(v.hi);
+    if (FULL) x += __mulhi(c.lo, v.lo);
   }
   __device__ __forceinline__ i64 result() const { return (hh << K) + ((x + x2) >> (32 - K)); }
 };
@@ -150,15 +152,20 @@ struct AccH {
   }
 };
 
-// v * 2^sh for 0 <= sh < 64: the operator's two renormalisation shifts are
-// never negative (values below 2^59; the FULL form has two bits more
-// everywhere).  After the gradient every output is below 2^59 (lx1
-// products of |C| <= 2^59 and an even-odd sum below 2^60, in units of 2^64,
-// lx1 <= 16), so its shift is >= 0; after the metric step every output is below
+// v * 2^sh for 0 <= sh < 64.  After the gradient every output is below 2^59
+// (lx1 products of |C| <= 2^59 and an even-odd sum below 2^60, in units of
+// 2^64, lx1 <= 16; two bits more everywhere in the FULL form), so its
+// renormalisation's shift is >= 0; after the metric step every output is below
 // 2^56.6 (three products of |G| < 2^60 and a value below 2^59), so its shift
-// is >= 2.  The operator checks both and reports a violation through the
+// is >= 2.  The FULL form's metric step leaves at most 3 * 2^61 (three products
+// of |G| and a value of at most 2^61, in units of 2^61): its shift is >= -2
+// (shift_to).  The operator checks both and reports a violation through the
 // device error word.
 __device__ __forceinline__ i64 shift_up(i64 v, int sh) { return i64(u64(v) << sh); }
+// the same for -2 <= sh, rounded to nearest
+__device__ __forceinline__ i64 shift_to(i64 v, int sh) {
+  return sh >= 0 ? shift_up(v, sh) : (v + (1ll << (-sh - 1))) >> -sh;
+}
 
 // ----------------------------------------------------- FP64 <-> fixed --
 __device__ __forceinline__ int bexp(double x) {
@@ -237,14 +244,15 @@ __device__ __forceinline__ i64 to_fixed_cvt(double x, int emax, int up) {
   const double sc = __longlong_as_double(i64(k + 1023) << 52);
   return __double2ll_rn(x * sc);
 }
-// x * 2^(1082 - emax) rounded to nearest (halves away from zero), |result| <=
-// 2^60, for x whose biased exponent is <= emax, on the integer pipes
-__device__ __forceinline__ i64 to_fixed60(double x, int emax) {
-  if (emax < 128) return to_fixed(x, emax, 7);  // (near the subnormals; uniform)
+// x * 2^(1022 + B - emax) rounded to nearest (halves away from zero), |result|
+// <= 2^B, for x whose biased exponent is <= emax, on the integer pipes
+template <int B>
+__device__ __forceinline__ i64 to_fixed_bits(double x, int emax) {
+  if (emax < 128) return to_fixed(x, emax, B - 53);  // (near the subnormals; uniform)
   const u64 b = u64(__double_as_longlong(x));
   const int e = int((b >> 52) & 0x7FFu);
   const int r = min(emax - e, 63);  // a zero (e = 0) shifts out
-  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << 8;
+  const u64 m = ((b & 0xFFFFFFFFFFFFFull) | (1ull << 52)) << (B - 52);
   const i64 v = i64(((m >> r) + 1ull) >> 1), s = i64(b) >> 63;
   return (v ^ s) - s;
 }
@@ -268,11 +276,16 @@ __device__ __forceinline__ unsigned warp_mask(int nt, int w) {
 // cross terms as high words (AccH); the matrix's other part, the rounding
 // (~1e-15) by which D misses the symmetry, is dropped.
 // Odd lx1 up to 11 (FULL): these orders' other form is the reference's own
-// FP64 sums, and this one is to be no less exact: |coefficient| <= 2^61 and
-// |line value| < 2^61, cross terms in full (AccF), and the centrosymmetric
-// remainder of D kept as one 32-bit coefficient more a product, in the unit
-// of lo (dE, h1 rows of h1 values, and dO, h rows of h):
-//   y(a) += dE ve + dO vo,  y(n-1-a) += dE ve - dO vo.
+// FP64 sums, and this one is no less exact: |coefficient| <= 2^61 and
+// |line value| < 2^61, cross terms in full (AccF), the metric to 61 bits and
+// its products' low halves too (Acc), and the centrosymmetric remainder of D
+// kept as one 32-bit coefficient more a product, in the unit of lo (dE, h1 rows
+// of h1 values, and dO, h rows of h):
+//   y(a) += dE ve + dO vo,  y(n-1-a) += dE ve - dO vo,
+// rounded to nearest: a floor takes half a unit off every point, and CG makes
+// much of a constant (x after 40 iterations at lx1 = 9, against quadruple
+// precision: 8.4e-16 with floors, 3.1e-16 so, 3.2e-16 with FP64 sums; with the
+// metric to 60 bits and its products' high halves alone 3.5e-16).
 // A kernel parameter, read as multiply-add operands.
 template <int LX>
 struct FxCoef {
@@ -288,6 +301,8 @@ struct FxCoef {
 // bits of a line's values: |v| < 2^kLine (and of a block after renormalising)
 template <int LX>
 constexpr int fx_bits() { return FxCoef<LX>::FULL ? 61 : 59; }
+// Bits of the metric's values: |G| <= 2^fx_gbits, of the element's largest.
+constexpr int fx_gbits(int lx) { return lx % 2 != 0 ? 61 : 60; }
 
 // ------------------------------------------------------ separable metric --
 // A box of equal cubes (setup_g, prox_setup.f:27-52) has the same block in
@@ -360,7 +375,7 @@ __device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int 
     for (int m = 0; m < H; ++m) o.mac(cf.hi[qo0 + a * H + m], cf.lo[qo0 + a * H + m], vo[m], m);
     const i64 ye = e.result(H1), yo = o.result(H);
     if constexpr (FULL) {
-      i64 ze = 0, zo = 0;
+      i64 ze = 1ll << 31, zo = 0;
 #pragma unroll
       for (int m = 0; m < H1; ++m) ze += i64(cf.d[de0 + a * H1 + m]) * i64(ve[m].hi);
 #pragma unroll
@@ -374,7 +389,7 @@ __device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int 
   }
   if constexpr (FULL) {  // the middle output
     A o;
-    i64 ze = 0;
+    i64 ze = 1ll << 31;
 #pragma unroll
     for (int m = 0; m < H; ++m)
       o.mac(cf.hi[qo0 + H * H + m], cf.lo[qo0 + H * H + m], vo[m], m);
@@ -427,6 +442,11 @@ __device__ __forceinline__ int fx_or_shift(const unsigned *orl, const unsigned *
   for (int w = 0; w < (nt + 31) / 32; ++w) v |= (u64(orh[w]) << 32) | orl[w];
   if (v == 0) return 0;
   return bits - 1 - (63 - __clzll(i64(v)));
+}
+// the second renormalisation of a value (shift_up)
+template <int LX>
+__device__ __forceinline__ i64 fx_shift2(i64 v, int sh) {
+  return FxCoef<LX>::FULL ? shift_to(v, sh) : shift_up(v, sh);
 }
 // one's complement magnitude: the same top bit as |v| (one lower for an
 // exact negative power of two, which the bounds leave room for)
@@ -556,7 +576,7 @@ __device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX
     for (int q = 0; q < (L2 + 31) / 32; ++q) em = max(em, sm.emax[q]);
     // (on the integer pipes: this form is held by the FP64 one)
 #pragma unroll
-    for (int k = 0; k < LX; ++k) sm.A[fx_at<LX>(i, j, k)] = to_fixed60(uk[k], em);
+    for (int k = 0; k < LX; ++k) sm.A[fx_at<LX>(i, j, k)] = to_fixed_bits<60>(uk[k], em);
   }
   __syncthreads();
 
@@ -608,7 +628,7 @@ template <int LX, int MODE>
 __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef<LX> &cf) {
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FxShared<LX> &sm = *reinterpret_cast<FxShared<LX> *>(smem_raw);
-  constexpr int L2 = LX * LX, L3 = LX * LX * LX, BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 2 : 0;
+  constexpr int L2 = LX * LX, L3 = LX * LX * LX, BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 3 : 0;
   const int t = threadIdx.x + LX * threadIdx.y;
   const int i = threadIdx.x, j = threadIdx.y;  // own column (i,j)
   const int e = blockIdx.x;
@@ -723,7 +743,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   } else {
     eg = a.gexp[e];
   }
-  const int sW = 64 - MK + (eg - 1082) + sU;  // wr = WR 2^sW before renormalising
+  const int sW = 64 - MK + (eg - 1022 - fx_gbits(LX)) + sU;  // wr = WR 2^sW before renormalising
   orv = 0;
 #pragma unroll 4
   for (int k = 0; k < LX; ++k) {
@@ -734,19 +754,19 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     if constexpr (MODE == 3) {
       const double2 *gp = reinterpret_cast<const double2 *>(a.g + 6 * (base + size_t(k) * L2 + t));
       const double2 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
-      G1 = split(to_fixed60(g01.x, eg));
-      G2 = split(to_fixed60(g01.y, eg));
-      G3 = split(to_fixed60(g23.x, eg));
-      G4 = split(to_fixed60(g23.y, eg));
-      G5 = split(to_fixed60(g45.x, eg));
-      G6 = split(to_fixed60(g45.y, eg));
+      G1 = split(to_fixed_bits<fx_gbits(LX)>(g01.x, eg));
+      G2 = split(to_fixed_bits<fx_gbits(LX)>(g01.y, eg));
+      G3 = split(to_fixed_bits<fx_gbits(LX)>(g23.x, eg));
+      G4 = split(to_fixed_bits<fx_gbits(LX)>(g23.y, eg));
+      G5 = split(to_fixed_bits<fx_gbits(LX)>(g45.x, eg));
+      G6 = split(to_fixed_bits<fx_gbits(LX)>(g45.y, eg));
     } else {
       const int4 *gp = reinterpret_cast<const int4 *>(a.gfx + 6 * (base + size_t(k) * L2 + t));
       const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
       G1 = Sp{g01.x, g01.y}, G2 = Sp{g01.z, g01.w}, G3 = Sp{g23.x, g23.y};
       G4 = Sp{g23.z, g23.w}, G5 = Sp{g45.x, g45.y}, G6 = Sp{g45.z, g45.w};
     }
-    Acc<MK> wr, ws, wt;
+    Acc<MK, FxCoef<LX>::FULL> wr, ws, wt;
     wr.mac(G1, ur); wr.mac(G2, us); wr.mac(G3, ut);
     ws.mac(G2, ur); ws.mac(G4, us); ws.mac(G5, ut);
     wt.mac(G3, ur); wt.mac(G5, us); wt.mac(G6, ut);
@@ -759,7 +779,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
   fx_or_post(orv, sm.orl[1], sm.orh[1], t, L2);
   __syncthreads();
   int s2 = fx_or_shift(sm.orl[1], sm.orh[1], L2, BITS);
-  if (s2 < 0) {  // as s1
+  if (s2 < (FxCoef<LX>::FULL ? -2 : 0)) {  // as s1
     if (t == 0 && a.err) atomicOr(a.err, 2u);
     s2 = 0;
   }
@@ -775,7 +795,7 @@ __device__ __forceinline__ void ax_fx_body(const AxArgs<double> &a, const FxCoef
     const i64 *src = out;
     i64 v[LX];
 #pragma unroll
-    for (int m = 0; m < LX; ++m) v[m] = shift_up(src[b0 + m * st], s2);
+    for (int m = 0; m < LX; ++m) v[m] = fx_shift2<LX>(src[b0 + m * st], s2);
     fx_line<LX>(v, cf, 1, [&](int m, i64 y) { out[b0 + m * st] = y; });
   }
   __syncthreads();
@@ -808,7 +828,7 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
   extern __shared__ __align__(128) unsigned char smem_raw[];
   FxShared<LX> &sm = *reinterpret_cast<FxShared<LX> *>(smem_raw);
   constexpr int L2 = LX * LX, L3 = LX * LX * LX, NTH = 3 * L2, NW = (NTH + 31) / 32;
-  constexpr int BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 2 : 0, NK = (LX + 2) / 3;
+  constexpr int BITS = fx_bits<LX>(), MK = FxCoef<LX>::FULL ? 3 : 0, NK = (LX + 2) / 3;
   constexpr bool SEP = !FxCoef<LX>::FULL;
   const int tid = threadIdx.x, grp = tid / L2, t = tid - grp * L2, i = t % LX, j = t / LX;
   const int e = blockIdx.x, w = tid >> 5, k0 = grp * NK;
@@ -846,7 +866,7 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
     for (int q = 0; q < NK; ++q) {
       if (k0 + q >= LX) break;
       sm.A[fx_at<LX>(i, j, k0 + q)] =
-          SEP && sep.x ? to_fixed60(uk[q], em) : to_fixed_cvt(uk[q], em, BITS - 53);
+          SEP && sep.x ? to_fixed_bits<60>(uk[q], em) : to_fixed_cvt(uk[q], em, BITS - 53);
     }
   }
   __syncthreads();
@@ -891,7 +911,7 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
       s1 = 0;
     }
     const int eg = a.gexp[e];
-    const int sW = 64 - MK + (eg - 1082) + (em - 1075 - (BITS - 53)) - cf.fc + 64 - s1;
+    const int sW = 64 - MK + (eg - 1022 - fx_gbits(LX)) + (em - 1075 - (BITS - 53)) - cf.fc + 64 - s1;
     orv = 0;
 #pragma unroll
     for (int k_ = 0; k_ < NK; ++k_) {
@@ -904,7 +924,7 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
       const int4 g01 = __ldg(gp), g23 = __ldg(gp + 1), g45 = __ldg(gp + 2);
       const Sp G1 = {g01.x, g01.y}, G2 = {g01.z, g01.w}, G3 = {g23.x, g23.y},
                G4 = {g23.z, g23.w}, G5 = {g45.x, g45.y}, G6 = {g45.z, g45.w};
-      Acc<MK> wr, ws, wt;
+      Acc<MK, FxCoef<LX>::FULL> wr, ws, wt;
       wr.mac(G1, ur); wr.mac(G2, us); wr.mac(G3, ut);
       ws.mac(G2, ur); ws.mac(G4, us); ws.mac(G5, ut);
       wt.mac(G3, ur); wt.mac(G5, us); wt.mac(G6, ut);
@@ -917,13 +937,13 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
     fx_or_post(orv, sm.orl[1], sm.orh[1], tid, NTH);
     __syncthreads();
     int s2 = fx_or_shift(sm.orl[1], sm.orh[1], NTH, BITS);
-    if (s2 < 0) {  // as s1
+    if (s2 < (FxCoef<LX>::FULL ? -2 : 0)) {  // as s1
       if (tid == 0 && a.err) atomicOr(a.err, 2u);
       s2 = 0;
     }
     const int sT = 64 - cf.fc + sW - s2;
 #pragma unroll
-    for (int m = 0; m < LX; ++m) v[m] = shift_up(out[b0 + m * st], s2);
+    for (int m = 0; m < LX; ++m) v[m] = fx_shift2<LX>(out[b0 + m * st], s2);
     fx_line<LX>(v, cf, 1, [&](int m, i64 y) { out[b0 + m * st] = y; });
     __syncthreads();
     const bool bad = em == 0x7FF || eg == 0x7FF;
