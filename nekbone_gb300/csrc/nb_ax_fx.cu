@@ -90,29 +90,25 @@ __device__ __forceinline__ DD dd_add(DD a, DD b) {
   return dd_sum(s.h, __dadd_rn(s.l, __dadd_rn(a.l, b.l)));
 }
 
-// K and its fixed-point tables from D and element 0's v, by one block:
-// K(i,m) in double-double for the upper rows i < h, then E and O, each the
-// nearest integer of the value times 2^fc.  Like the even-odd tables of the
-// general form it takes D's upper rows and their mirror images; b is made
-// symmetric (K then is).  False where a sum of the operator's accumulators
-// (Acc, and the three directions) could leave 64 bits.
+__device__ __forceinline__ DD dd_sub(DD a, DD b) { return dd_add(a, DD{-b.h, -b.l}); }
+
+// K and its tables from D and element 0's v, by one block: K(i,m) in
+// double-double, then E and O, each the nearest integer of the value times
+// 2^fc, and the rest.  False where a sum of the operator's accumulators (Acc,
+// and the three directions) could leave 64 bits, or the rest's 24.
 __device__ bool sep_tables(const double *__restrict__ D, int lx, fx::SepTables *sep) {
-  __shared__ DD K[128];
+  __shared__ DD K[256];
   __shared__ double bs[16];
   __shared__ int emax[8];
-  const int t = threadIdx.x, h = lx / 2, n1 = lx - 1, nk = h * lx;
-  if (t < lx) {
-    const int at = lx * h + lx * lx * h;
-    bs[t] = 0.5 * (sep->v[t + at] + sep->v[n1 - t + at]);
-  }
+  const int t = threadIdx.x, h = lx / 2, n1 = lx - 1, nk = lx * lx;
+  if (t < lx) bs[t] = sep->v[t + lx * h + lx * lx * h];
   __syncthreads();
   int em = 0;
   if (t < nk) {
     const int i = t / lx, m = t % lx;
-    auto Du = [&](int r, int c) { return r < h ? D[r + c * lx] : -D[n1 - r + (n1 - c) * lx]; };
     DD k = {0.0, 0.0};
     for (int q = 0; q < lx; ++q) {
-      const double a = Du(q, i), b = Du(q, m), w = bs[q];
+      const double a = D[q + i * lx], b = D[q + m * lx], w = bs[q];
       const double p = __dmul_rn(a, b), pe = __fma_rn(a, b, -p);  // a b = p + pe
       const double r = __dmul_rn(p, w), re = __fma_rn(pe, w, __fma_rn(p, w, -r));
       const DD x = dd_sum(k.h, r);
@@ -124,12 +120,17 @@ __device__ bool sep_tables(const double *__restrict__ D, int lx, fx::SepTables *
   }
   __syncthreads();
   // value t of the tables, and the largest exponent among them
-  DD p = {0.0, 0.0};
-  if (t < 2 * h * h) {
-    const int a = (t % (h * h)) / h, c = t % h;
-    const double s = t < h * h ? 0.5 : -0.5;  // E, O
-    const DD x = K[a * lx + c], y = K[a * lx + n1 - c];
-    p = dd_add(DD{0.5 * x.h, 0.5 * x.l}, DD{s * y.h, s * y.l});
+  DD p = {0.0, 0.0}, rest = {0.0, 0.0};
+  const int at = t % (h * h), which = t / (h * h);  // which: 0 E, 1 O
+  if (which < 2) {
+    const int a = at / h, c = at % h;
+    const DD k00 = K[a * lx + c], k01 = K[a * lx + n1 - c];
+    const DD k10 = K[(n1 - a) * lx + c], k11 = K[(n1 - a) * lx + n1 - c];
+    const DD x = dd_add(k00, k11), y = dd_add(k01, k10);
+    const DD u = dd_sub(k00, k11), w = dd_sub(k01, k10);
+    p = which ? dd_sub(x, y) : dd_add(x, y);
+    rest = which ? dd_sub(u, w) : dd_add(u, w);
+    p = {0.25 * p.h, 0.25 * p.l};
     em = fx::bexp(p.h);
   }
   em = int(__reduce_max_sync(0xFFFFFFFFu, unsigned(em)));
@@ -138,28 +139,32 @@ __device__ bool sep_tables(const double *__restrict__ D, int lx, fx::SepTables *
   for (int q = 0; q < 8; ++q) em = max(em, emax[q]);
   const int fc = 61 - (em - 1022);  // every value below 2^(em - 1022)
   bool good = em > 1 && em < 2046;
-  if (good && t < 2 * h * h) {
+  if (good && which < 2) {
     // the high part times 2^fc has a fraction of at most 52 bits: both exact
     const double hs = scalbn(p.h, fc), hi = rint(hs);
     const long long C = (long long)hi + __double2ll_rn((hs - hi) + scalbn(p.l, fc));
     const fx::Sp sp = fx::split(C);
-    sep->tab[t] = make_int2(sp.hi, sp.lo);
+    reinterpret_cast<int2 *>(sep->tab)[2 * at + which] = make_int2(sp.hi, sp.lo);
+    reinterpret_cast<float *>(sep->rest)[2 * at + which] =
+        float(scalbn(0.25 * (rest.h + rest.l), fc - 32));
     good = C <= (1ll << 61) && C >= -(1ll << 61);
   }
   __syncthreads();
   if (good && t < h) {  // the rows' sums
-    double xe = 0.0, xo = 0.0, hm = 0.0;
+    double xe = 0.0, xo = 0.0, hm = 0.0, rm = 0.0;
     for (int c = 0; c < h; ++c) {
-      const int2 e = sep->tab[t * h + c], o = sep->tab[h * h + t * h + c];
-      const double ae = fabs(double(e.x)) + 1.0, ao = fabs(double(o.x)) + 1.0;
+      const int4 eo = sep->tab[t * h + c];
+      const float2 d = sep->rest[t * h + c];
+      const double ae = fabs(double(eo.x)) + 1.0, ao = fabs(double(eo.z)) + 1.0;
       // x + x2 of a sum, in units of 2^31: |hi| 2^31 + |lo| 2^29 a term
-      xe += ae + 0.25 * fabs(double(e.y));
-      xo += ao + 0.25 * fabs(double(o.y));
+      xe += ae + 0.25 * fabs(double(eo.y));
+      xo += ao + 0.25 * fabs(double(eo.w));
       hm += fmax(ae, ao);
+      rm += fabs(double(d.x)) + fabs(double(d.y));
     }
     // the output: three directions of at most sum max(|E|, |O|) times 2^61, in
-    // units of 2^64
-    good = xe < 4.29e9 && xo < 4.29e9 && 3.0 * hm < 1.7e10;
+    // units of 2^64; the rest: values' high halves of at most 2^29
+    good = xe < 4.29e9 && xo < 4.29e9 && 3.0 * hm < 1.7e10 && rm * 0x1p29 < 0x1p24;
   }
   if (t == 0) sep->fc = fc;
   return good;
@@ -196,8 +201,9 @@ __global__ void __launch_bounds__(256)
         const double v = g[6 * l];
         const double a = line(l % lx), b = line((l / lx) % lx), c = line(l / L2);
         const double l1 = v * gm * gm, l2 = a * b * c;
-        // (2e-15: up to eight roundings on each side); b symmetric to 2e-14:
-        // zwgll's own weights differ by 6e-15 at lx1 = 12 and 1.2e-14 at 16
+        // (2e-15: up to eight roundings on each side); b symmetric to 2e-14, so
+        // that the rest is small: zwgll's own weights differ by 6e-15 at lx1 =
+        // 12 and 1.2e-14 at 16
         ok &= v > 1e-60 && v < 1e60 && fabs(l1 - l2) <= 2e-15 * l2;
         ok &= fabs(a - line(lx - 1 - l % lx)) <= 2e-14 * a;
         sep->v[l] = v;

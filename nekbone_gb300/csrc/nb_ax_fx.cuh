@@ -313,21 +313,30 @@ constexpr int fx_gbits(int lx) { return lx % 2 != 0 ? 61 : 60; }
 // six, no metric step and no metric read but one shared block.  k_sep_check
 // establishes the form on the device, once per solve, from g itself (every
 // element bitwise, the product to the rounding of its factors), and makes K in
-// double-double.  ok = 0: the general form.
+// double-double from D and b as they are.  ok = 0: the general form.
+// K is centrosymmetric but for the rounding (~1e-14) by which D and b miss
+// their symmetry.  The centrosymmetric part is E and O, h x h each (row a),
+// |coefficient| <= 2^61; the rest, dE and dO, is added in FP32, which has 24
+// bits of it to spare and whose pipe is idle:
+//   y(a) = E ve + O vo + dE ve + dO vo,  y(n-1-a) = E ve - O vo - dE ve + dO vo.
+// Without the rest and with b made symmetric an apply was off by 2.7e-15 at
+// lx1 = 12 and 5.5e-15 at 16 (random field, 2-norm against quadruple
+// precision), with it 1.2e-16 and 1.4e-16, as the FP64 sums; x after 40
+// iterations at lx1 = 12 by 2.7e-15 and 3.7e-16.
 struct SepTables {
   int ok, fc;        // fc: fractional bits of the tables
   int pad[2];
-  // (hi, lo) of E, then of O, h x h each (row a), |coefficient| <= 2^61; K is
-  // centrosymmetric: y(a) = E ve + O vo, y(n-1-a) = E ve - O vo
-  int2 tab[2 * 64];
+  int4 tab[64];      // (hi, lo) of E, (hi, lo) of O
+  float2 rest[64];   // dE, dO in units of 2^(32 - fc)
   double v[4096];
 };
 
 template <int LX>
 struct FxShared {
   static constexpr int N = (LX * LX + 1) * LX;
-  static constexpr int NT = FxCoef<LX>::FULL ? 2 : 2 * (LX / 2) * (LX / 2);
-  alignas(16) int2 tab[NT];  // SepTables' tables
+  static constexpr int NT = FxCoef<LX>::FULL ? 1 : (LX / 2) * (LX / 2);
+  alignas(16) int4 tab[NT];  // SepTables' tables
+  float2 rest[NT];
   i64 A[N];
   i64 C[N];
   i64 D[N];
@@ -401,26 +410,34 @@ __device__ __forceinline__ void fx_line(const i64 *v, const FxCoef<LX> &cf, int 
 
 // y = K v of one line, |v| < 2^60 (SepTables)
 template <int LX, typename Put>
-__device__ __forceinline__ void fx_line_sep(const i64 *v, const int2 *tab, Put put) {
+__device__ __forceinline__ void fx_line_sep(const i64 *v, const int4 *tab, const float2 *rest,
+                                            Put put) {
   constexpr int H = LX / 2;
   Sp ve[H], vo[H];
+  float fe[H], fo[H];
 #pragma unroll
   for (int m = 0; m < H; ++m) {
     ve[m] = split(v[m] + v[LX - 1 - m]);
     vo[m] = split(v[m] - v[LX - 1 - m]);
+    fe[m] = float(ve[m].hi);
+    fo[m] = float(vo[m].hi);
   }
 #pragma unroll 1
   for (int a = 0; a < H; ++a) {
     Acc<0> e, o;
+    float ze = 0.f, zo = 0.f;
 #pragma unroll
     for (int m = 0; m < H; ++m) {
-      const int2 ce = tab[a * H + m], co = tab[H * H + a * H + m];
-      e.mac(Sp{ce.y, ce.x}, ve[m]);
-      o.mac(Sp{co.y, co.x}, vo[m]);
+      const int4 c = tab[a * H + m];
+      const float2 d = rest[a * H + m];
+      e.mac(Sp{c.y, c.x}, ve[m]);
+      o.mac(Sp{c.w, c.z}, vo[m]);
+      ze = fma_rn(d.x, fe[m], ze);
+      zo = fma_rn(d.y, fo[m], zo);
     }
     const i64 ye = e.result(), yo = o.result();
-    put(a, ye + yo);
-    put(LX - 1 - a, ye - yo);
+    put(a, ye + yo + i64(__float2int_rn(zo + ze)));
+    put(LX - 1 - a, ye - yo + i64(__float2int_rn(zo - ze)));
   }
 }
 
@@ -517,13 +534,13 @@ __device__ __forceinline__ double ax_fx_finish(const AxArgs<double> &a, int e, i
 // The operator where SepTables' form holds (MODE 1 and 2 as ax_fx_body).  Two
 // of the shared arrays: the element in fixed point (A), and the sum of the
 // three directions' results (C), each direction's lines added by the threads
-// that own them.  About 300 instructions a point at half an issue a cycle and
-// five FP64 operations (58 % of that pipe): 0.86 ms at 32^3, lx1 = 12, against
-// 1.53 for the general form.  Measured and left out: the result's conversion
-// and product on the integer pipes (40 instructions for two FP64 operations,
-// 0.88 to 0.95 ms); two elements a CTA (0.88); a kernel of its own with six
-// CTAs per SM (0.81 to 0.86, but 3 to 6 us a launch on small meshes, since
-// the device decides which of the two runs).
+// that own them.  1.00 ms at 32^3, lx1 = 12, against 1.53 for the general
+// form, 0.10 of it for K's part that is not centrosymmetric (SepTables).
+// Measured without that part, 0.86 ms then, and left out: the result's
+// conversion and product on the integer pipes (40 instructions for two FP64
+// operations, 0.88 to 0.95 ms); two elements a CTA (0.88); a kernel of its own
+// with six CTAs per SM (0.81 to 0.86, but 3 to 6 us a launch on small meshes,
+// since the device decides which of the two runs).
 template <int LX, int MODE>
 __device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX> &sm, bool whole,
                                             unsigned nbr, int fc) {
@@ -532,7 +549,10 @@ __device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX
   const int i = threadIdx.x, j = threadIdx.y;  // own column (i,j)
   const int e = blockIdx.x;
   const size_t base = size_t(e) * L3;
-  if (t < NT) sm.tab[t] = a.sep->tab[t];
+  if (t < NT) {
+    sm.tab[t] = a.sep->tab[t];
+    sm.rest[t] = a.sep->rest[t];
+  }
 
   int em = 0;
   {
@@ -590,7 +610,7 @@ __device__ __forceinline__ void ax_sep_body(const AxArgs<double> &a, FxShared<LX
     i64 v[LX];
 #pragma unroll
     for (int m = 0; m < LX; ++m) v[m] = sm.A[b0 + m * st];
-    fx_line_sep<LX>(v, sm.tab, [&](int m, i64 y) {
+    fx_line_sep<LX>(v, sm.tab, sm.rest, [&](int m, i64 y) {
       i64 *o = sm.C + b0 + m * st;
       *o = d ? *o + y : y;
     });
@@ -836,7 +856,10 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
   const bool whole = box_flag(a.box_ok);
   const unsigned nbr = whole ? box_neighbours(a.box, e) : 0u;
   const int2 sep = SEP && a.sep ? *reinterpret_cast<const int2 *>(a.sep) : make_int2(0, 0);
-  if (SEP && sep.x && tid < FxShared<LX>::NT) sm.tab[tid] = a.sep->tab[tid];
+  if (SEP && sep.x && tid < FxShared<LX>::NT) {
+    sm.tab[tid] = a.sep->tab[tid];
+    sm.rest[tid] = a.sep->rest[tid];
+  }
   const unsigned lanes = warp_mask(NTH, w);
   int em = 0;
   {
@@ -883,7 +906,7 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
   bool done = false;
   if constexpr (SEP) {
     if (sep.x) {
-      fx_line_sep<LX>(v, sm.tab, [&](int m, i64 y) { out[b0 + m * st] = y; });
+      fx_line_sep<LX>(v, sm.tab, sm.rest, [&](int m, i64 y) { out[b0 + m * st] = y; });
       __syncthreads();
       const int sY = em - 1075 - (60 - 53) + 64 - sep.y;
       const bool bad = em == 0x7FF;
