@@ -981,8 +981,12 @@ __device__ __forceinline__ void ax_fx_wide(const AxArgs<double> &a, const FxCoef
   if (tid == 0) a.partial[e] = s;
 }
 
+// (resident CTAs asked for at 10 and 12: the separable form's line would take 88
+// and 114 registers there, and 20 CG iterations at lx1 = 12, box / deformed, on
+// 6^3 elements 767 / 916 us instead of 676 / 810; elsewhere the bound has no or
+// the opposite effect)
 template <int LX>
-__global__ void __launch_bounds__((3 * LX * LX + 31) / 32 * 32)
+__global__ void __launch_bounds__((3 * LX * LX + 31) / 32 * 32, LX == 10 ? 3 : LX == 12 ? 2 : 0)
     k_ax_fx_wide(AxArgs<double> a, const __grid_constant__ FxCoef<LX> cf) {
   dependent_begin();
   ax_fx_wide<LX>(a, cf);
