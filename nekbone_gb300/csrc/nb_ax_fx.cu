@@ -328,7 +328,7 @@ int metric_fx_prepare(const Operator &op, const double *g, const double *D, bool
   op.sep_on = sep;
   if (sep) {
     NB_CUDA(cudaMemsetAsync(&op.sep->ok, 1, sizeof(int), s));
-    k_sep_check<<<std::min(op.nelt, 152 * 8), 256, 0, s>>>(g, D, op.lx, op.nelt, op.sep);
+    k_sep_check<<<std::min(op.nelt, sm_count() * 8), 256, 0, s>>>(g, D, op.lx, op.nelt, op.sep);
   }
   k_metric_fx<<<op.nelt, 256, 0, s>>>(g, op.gfx, op.gexp, blk, fx::fx_gbits(op.lx),
                                        sep ? op.sep : nullptr);

@@ -8,18 +8,28 @@
 namespace nb {
 
 // Where the CG pass takes three threads a column (k_ax_fx_wide).  20 CG
-// iterations, box / deformed, one thread -> three: small elements fill their
-// warps at any size (lx1 = 4 on 20^3: 900 / 1008 -> 795 / 901 us; 6 on 24^3:
-// 2707 / 3509 -> 2344 / 2916; 9 on 16^3: 3325 -> 3136), others while the mesh
-// does not fill the SMs (8 on 8^3: 573 / 635 -> 557 / 622, on 16^3: 1491 / 1927
-// -> 1553 / 2114; 10 on 810 elements: 970 / 1226 -> 946 / 1197, on 20^3: 4832 /
-// 6694 -> 4973 / 7465; 12 on 6^3: 736 / 926 -> 673 / 818, on 8^3: 1050 / 1399 ->
-// 1062 / 1354; 14 on 125: 734 / 860 -> 700 / 815, on 216: 947 / 1225 -> 1031 /
-// 1285).
+// iterations in us, box / deformed (odd lx1: one figure, the form is the same),
+// one thread -> three.  Small elements fill their warps at any size:
+//   lx1  4: 64 elements 329 / 339 -> 307 / 312; 20^3 906 / 1003 -> 795 / 889
+//        5: 27 376 -> 330; 8^3 456 -> 432; 20^3 1440 -> 1455
+//        6: 6^3 377 / 402 -> 343 / 352; 24^3 2686 / 3487 -> 2368 / 2926
+//        7: 27 438 -> 369; 8^3 636 -> 604; 18^3 2436 -> 2361
+//        9: 27 490 -> 403; 9^3 1044 -> 928; 24^3 9968 -> 9650
+// Others gain while the mesh does not fill the SMs:
+//        8: 600 589 / 645 -> 577 / 630; 704 619 / 705 -> 655 / 706; 16^3 1496 /
+//           1924 -> 1658 / 2239
+//       10: 64 461 / 504 -> 428 / 457; 10^3 1101 / 1388 -> 1099 / 1394; 20^3 4913
+//           / 6674 -> 5197 / 7490
+//       11: 27 550 -> 489; 304 850 -> 837; 8^3 1194 -> 1248; 14^3 3946 -> 4738
+//       12: 64 577 / 626 -> 491 / 547; 304 822 / 963 -> 741 / 874; 8^3 1075 / 1383
+//           -> 1083 / 1366
+//       14: 27 622 / 721 -> 581 / 672; 150 772 / 870 -> 733 / 826; 6^3 988 / 1223
+//           -> 1066 / 1285
+//       16: nothing (27 725 / 847 -> 725 / 851; 150 893 / 1033 -> 897 / 1035)
 inline bool ax_fx_is_wide(int lx, int nelt) {
-  if (lx < 4) return false;
+  if (lx < 4 || lx > 14) return false;
   if (lx <= 7 || lx == 9) return true;
-  return nelt <= (lx == 8 ? 600 : lx == 10 ? 1000 : lx <= 12 ? 304 : 152);
+  return nelt <= sm_count() * (lx == 8 ? 4 : lx == 10 ? 6 : lx <= 12 ? 2 : 1);
 }
 
 template <int LX, int MODE>
@@ -42,7 +52,7 @@ int launch_ax_fx_shape(const Operator &op, AxArgs<double> a, cudaStream_t s) {
   }
   for (int q = 0; q < Coef::QD; ++q) cf.d[q] = Coef::FULL ? op.FXd[q] : 0;
   cf.fc = op.fx_fc;
-  if constexpr (MODE == 1) {
+  if constexpr (MODE == 1 && LX >= 4 && LX <= 14) {
     if (ax_fx_is_wide(LX, a.nelt)) {
       static bool wide_set = false;
       if (!wide_set) {

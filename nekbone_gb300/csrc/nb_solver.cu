@@ -85,7 +85,7 @@ int CgWork::ensure_scratch(size_t bytes) {
   return NB_OK;
 }
 
-static int sm_count() {
+int sm_count() {
   static int cached = 0;
   if (!cached) {
     int dev = 0;
@@ -647,7 +647,7 @@ namespace {
 template <typename T>
 bool update_one_pass(const Operator &op) {
   const long n = sizeof(T) == 8 ? 200000 : 600000;
-  return op.n <= n || (op.nelt < 152 && op.n <= 600000);
+  return op.n <= n || (op.nelt < sm_count() && op.n <= 600000);
 }
 
 // k_cg_update_box in one form: its grid is one wave of resident blocks

@@ -178,6 +178,7 @@ int operator_set_mask(Operator *op, const std::vector<int> &list);
 std::vector<int> full_mask_list(const Operator &op);
 
 // ------------------------------------------------------------- kernels --
+int sm_count();  // SMs of the device
 // A launch on s that may start before the one before it has finished: for
 // kernels that begin with dependent_begin().
 template <typename... P, typename... A>
