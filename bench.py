@@ -50,9 +50,11 @@ UNIT = "GDOF*iter/s"
 # DRAM read + write bytes per point of each FP64 element operator at lx1 = 12
 # from one ncu capture on 16^3 elements (7,077,888 points); the kernels
 # stream, so traffic scales with n.  Source: the profiles/ summaries named.
+# (Order 2 takes the separable form on the benchmark's box; at 16^3 a fifth of
+# what it writes is still in L2 when the capture ends.)
 DRAM_BYTES_PER_POINT = {
     1: ((531.699456e6 + 120.930048e6) / 7077888, "profiles/k_ax_eo_fp64_lx12_16cubed.md"),
-    2: ((511.710208e6 + 98.418944e6) / 7077888, "profiles/k_ax_fx_fp64_lx12_16cubed.md"),
+    2: ((113.333760e6 + 67.918592e6) / 7077888, "profiles/k_ax_sep_fp64_lx12_16cubed.md"),
 }
 RHS_SEED = 20260
 
@@ -536,8 +538,9 @@ def run_ours(a, rank, world, local):
     unique = ((lx - 1) * nel + 1) ** 3
     clocks = clk.summary()
     ms_per_step = ms / a.steps
-    # per step: x = 0 / r = mask(f) / r'Cr (3), the fixed-point metric (order 2),
-    # then 3 kernels per iteration
+    # per step: order 2 the start (x, r, r'Cr and the box check), the metric's
+    # two kernels, 3 kernels per iteration and the last w finished; the others
+    # r = f, its mask and r'Cr, then 3 kernels per iteration
     launches_per_step = 3 + (1 if order == 2 else 0) + 3 * niter
     x100 = _host(x) if rank == 0 and world == 1 and not a.no_cpu else None
 
@@ -549,14 +552,18 @@ def run_ours(a, rank, world, local):
         kms[o] = mesh.time_cg_kernels(x.data_ptr(), f.data_ptr(), g.data_ptr(), c.data_ptr(),
                                       r.data_ptr(), w.data_ptr(), p.data_ptr(), reps=10)
     mesh.set_order(order)
-    ax_bytes = 64 * n   # u 8 + g 48 + w 8 per point (ax, stored metric)
+    # bytes per point: with a stored metric u 8 + g 48 + w 8 (ax); the separable
+    # form, which the box takes at order 2 and even lx1, reads no metric: r and
+    # the old direction 16, the direction and w written 16
+    sep = order == 2 and lx % 2 == 0
+    ax_bytes = (32 if sep else 64) * n
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
     peak = float(peaks.get("hbm_gbs", 6800.0))
     rates = nb.pipe_rates()
     achieved = ax_bytes / (kms[order][0] * 1e-3) / 1e9
     flops_pt = 19 + 12 * lx
     names = {2: f"k_ax_fx<{lx},1> (fused FP64 element operator in 64-bit fixed point on the "
-                f"integer pipes, even-odd contractions)",
+                f"integer pipes, {'separable metric' if sep else 'even-odd contractions'})",
              1: f"k_ax_eo4<double,{lx},1> (fused FP64 element operator, even-odd contractions "
                 f"on the FP64 pipe)",
              0: f"k_ax_impl<double,{lx},1,false> (fused FP64 element operator, reference order)"}
@@ -566,11 +573,9 @@ def run_ours(a, rank, world, local):
                 "traffic": trf[0] * n if trf else None,
                 "traffic_source": trf[1] if trf else None,
                 "kernel": names[order],
-                "algorithmic_bytes_per_point": 64,
-                # a box of equal cubes takes the separable form inside the
-                # kernel, which checks the metric once a solve and then reads
-                # none of its 48 B a point
-                "bytes_note": "ax with a stored metric; the separable form reads no metric",
+                "algorithmic_bytes_per_point": ax_bytes // n,
+                "bytes_note": "separable metric: no metric read" if sep
+                              else "ax with a stored metric",
                 "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback",
                 "kernel_ms": {"ax": kms[order][0], "gs_fin": kms[order][1],
                               "update": kms[order][2]},

@@ -364,7 +364,7 @@ void *nb_stream(void);
  * pap, [2] x/r update and rtr -- over reps iterations (over 2 reps with
  * the paired x update of nb_set_paired_update, its two update forms
  * averaged), timed with CUDA events on the library stream.  Where the update
- * sums the copies itself (a full-mask box whose c and f pass the check), [1]
+ * sums the copies itself (a box whose c and f pass the check), [1]
  * only forms pap and alpha, and [2] holds the gather-scatter.  Vectors as for
  * nb_cg; x and r are overwritten. */
 int nb_time_cg_kernels(nb_mesh *mesh, double *x, const double *f,

@@ -40,8 +40,8 @@
 //    scaling and the FP64-to-integer conversion (two more), where the FP64
 //    pipe has room beside the integer work.
 // Odd lx1 up to 11 takes a form with more bits (FxCoef): 50 CG iterations on
-// 12 x 10 x 9 elements at lx1 = 9 in 4.28 ms instead of 9.07 with the
-// reference-order operator on the FP64 pipe.
+// 12 x 10 x 9 elements at lx1 = 9 in 2.96 ms, 9.05 with the reference-order
+// operator on the FP64 pipe (4.28 when the operator alone had changed).
 // This is block floating point: the error of a value is bounded relative to
 // the largest value of its element (~2^-56), where FP64 bounds it relative
 // to the value itself.  Results agree with the reference's FP64 evaluation
