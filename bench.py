@@ -50,8 +50,8 @@ UNIT = "GDOF*iter/s"
 # DRAM read + write bytes per point of each FP64 element operator at lx1 = 12
 # from one ncu capture on 16^3 elements (7,077,888 points); the kernels
 # stream, so traffic scales with n.  Source: the profiles/ summaries named.
-# (Order 2 takes the separable form on the benchmark's box; at 16^3 a fifth of
-# what it writes is still in L2 when the capture ends.)
+# (Order 2 takes the separable form on the benchmark's box; at 16^3 two fifths of
+# what it writes are still in L2 when the capture ends.)
 DRAM_BYTES_PER_POINT = {
     1: ((531.699456e6 + 120.930048e6) / 7077888, "profiles/k_ax_eo_fp64_lx12_16cubed.md"),
     2: ((113.333760e6 + 67.918592e6) / 7077888, "profiles/k_ax_sep_fp64_lx12_16cubed.md"),
